@@ -550,15 +550,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pr::kThreads, 1) spa
         }
         qslots += 2;
       }
+      // Lane l looks up key 8 pw + (l & 7) of this CTA's 32 keys of a tile.  The look-up is a chain of two loads that may each
+      // miss every cache (index list, block table): the index is loaded two tiles ahead and the row number formed one tile
+      // ahead, so that neither latency sits in the per-tile period of these warps (paged decode of 64 sequences, whole call:
+      // 78.5 -> 69.8 us; prefill, whose lists come from L2, unchanged).
+      auto load_idx = [&](int it) {
+        const int slot = it < nvt ? tile_list[qp * kMaxTiles + it] * kBK + static_cast<int>(rank) * kKeys + pw * 8 + (lane & 7) : p.topk;
+        return slot < p.topk ? __ldg(ctx.idx_row + slot) : -1;
+      };
+      // row number inside kv, -1 for a key that does not take part: it is fetched with a source size of zero, which fills
+      // the destination with zeros
+      auto row_of = [&](int idx) { return index_valid(ctx, idx) ? static_cast<int>(kv_row(p, ctx.b, idx)) : -1; };
+      int idx_next = load_idx(0);
+      int row_next = row_of(idx_next);
+      idx_next = load_idx(1);
       for (int it = 0; it < nvt; ++it, ++g) {
-        const int tile = tile_list[qp * kMaxTiles + it], s = (g + qslots) % kStages;
-        // the row numbers are fetched before the wait for the stage, so their latency is hidden behind it: lane l looks up
-        // key 8 pw + (l & 7) of this CTA's 32 keys
-        const int slot = tile * kBK + static_cast<int>(rank) * kKeys + pw * 8 + (lane & 7);
-        const int my_idx = slot < p.topk ? __ldg(ctx.idx_row + slot) : -1;
-        // row number inside kv, -1 for a key that does not take part: it is fetched with a source size of zero, which fills
-        // the destination with zeros
-        const int my_row = index_valid(ctx, my_idx) ? static_cast<int>(kv_row(p, ctx.b, my_idx)) : -1;
+        const int s = (g + qslots) % kStages;
+        const int my_row = row_next;
+        row_next = row_of(idx_next);
+        idx_next = load_idx(it + 2);
         if (g + qslots >= kStages && ok) ok = mbar_wait<true>(bar(kBarKvEmpty + s), (((g + qslots) / kStages) + 1) & 1, p.status);
         if (!ok) continue;
         const uint32_t stage = sBase + s * kStageBytes;
