@@ -291,3 +291,39 @@ def test_long_key_cache_131072_keys():
         got = idx[0, t, 0].numpy()
         assert set(got.tolist()) == set(ref_i[0].tolist())
         np.testing.assert_allclose(val[0, t, 0].numpy(), ref_v[0], rtol=2e-5, atol=2e-4)
+
+
+@pytest.mark.parametrize("B,S1,N1,S2,paged", [(3, 1, 64, 9000, True), (2, 2, 64, 3333, True), (2, 3, 64, 2050, False), (5, 1, 32, 1025, False),
+                                              (1, 1, 64, 127, False), (2, 4, 32, 20000, False), (1, 9, 8, 1152, True), (1, 128, 64, 4100, False)])
+def test_few_queries_over_chunks_of_keys(B, S1, N1, S2, paged, monkeypatch):
+    """The narrow kernel shapes (64 and 128 rows of queries x heads) and keys split over several CTAs, with ragged lengths whose
+    last chunks are empty: scores against the oracle (same tolerance as above), TMA and cp.async producers."""
+    import tilelang_ascend_b200 as dsa
+    q, k, w = orc.make_indexer_inputs(B, S1, S2, N1, 128, seed=B * 1000 + S1)
+    ak = torch.tensor([max(S1, S2 - 1013 * b) for b in range(B)], dtype=torch.int32)
+    aq = torch.full((B,), S1, dtype=torch.int32)
+    ref = np.full((B, S1, S2), -np.inf, dtype=np.float32)
+    for b in range(B):
+        n = int(ak[b])
+        ref[b, :, :n] = orc.indexer_scores(q[b:b + 1], k[b:b + 1, :n], w[b:b + 1], sparse_mode=3).numpy()[0]
+    for no_tma in ("0", "1"):
+        monkeypatch.setenv("DSA_INDEXER_NO_TMA", no_tma)
+        got = dsa.indexer_scores_raw(q.cuda(), k.cuda(), w.cuda(), sparse_mode=3, q_len_b=aq.cuda(), k_len_b=ak.cuda())
+        check_status()
+        _scores_close(got.cpu().numpy(), ref)
+        K = min(64, S2)
+        dense = dsa.lightning_indexer(q.cuda(), k.cuda(), w.cuda(), actual_seq_lengths_query=aq, actual_seq_lengths_key=ak, sparse_count=K)[0]
+        same, rows = topk_three_step(dense.cpu().numpy().reshape(B * S1, K), orc.topk_select(ref.reshape(B * S1, S2), K), ref.reshape(B * S1, S2), K)
+        assert same >= rows - 1
+        if paged:   # the same keys through a shuffled block table
+            bs = 32
+            nb = -(-S2 // bs)
+            perm = torch.randperm(B * nb, generator=torch.Generator().manual_seed(1)).to(torch.int32).view(B, nb)
+            pool = torch.zeros((B * nb, bs, 1, 128), dtype=k.dtype)
+            pad = torch.zeros((B, nb * bs, 1, 128), dtype=k.dtype)
+            pad[:, :S2] = k
+            pool[perm.long().view(-1)] = pad.view(B * nb, bs, 1, 128)
+            got_p = dsa.lightning_indexer(q.cuda(), pool.cuda(), w.cuda(), actual_seq_lengths_query=aq, actual_seq_lengths_key=ak,
+                                          block_table=perm, layout_key="PA_BSND", sparse_count=K)[0]
+            assert torch.equal(got_p, dense)
+        check_status()

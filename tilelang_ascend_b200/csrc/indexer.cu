@@ -6,13 +6,18 @@
 // follow cpu_lightning_indexer, examples/deepseek_v4/lightning_indexer.py:303-314.
 //
 // Tensor-core kernel (D = 128): the MMA is issued transposed -- A = a tile of 128 keys x 128 dims
-// (UMMA M = keys), B = (QB queries x N1 heads = 256 rows) x 128 dims -- so the TMEM accumulator has
+// (UMMA M = keys), B = (QB queries x N1 heads = 64, 128 or 256 rows) x 128 dims -- so the TMEM accumulator has
 // one key per lane and all heads of a query in consecutive columns.  The ReLU, the per-head weight
 // and the sum over heads are then a per-thread reduction over columns, and a warp writes 32
-// consecutive keys of one query row (coalesced).  Two accumulators (2 x 256 TMEM columns) let the
+// consecutive keys of one query row (coalesced).  Two accumulators (2 x kN TMEM columns) let the
 // reduction of tile i overlap the MMAs of tile i+1.  Key tiles are dense (128 consecutive keys x 128 dims): one thread
 // fetches each with two TMA tile loads (64 dims x 128 keys, 128-byte swizzle) into a 3-stage ring; when no tensor
 // map could be made for k (unaligned pointer) four warps fetch the tiles with cp.async instead.
+//
+// A batch entry with few queries (decode) takes a narrower B operand, and its keys are split over as many CTAs as fill the
+// chip: one CTA per sequence, 256 columns wide, left 116 of 148 SMs idle and spent three quarters of its reduction on queries
+// that do not exist (32 sequences of up to 49152 paged keys, 64 heads, whole lightning_indexer call with its selector and
+// host reads: 479 -> 214 us; 4096 queries x 8192 keys, whole call: 736 -> 707 us).
 //
 // Generic kernel (any D, any N1): CUDA-core fp32.
 #include <cuda.h>
@@ -42,43 +47,60 @@ __device__ __forceinline__ int indexer_limit(const IndexerParams& p, int b, int 
 namespace itc {
 constexpr int kD = 128;
 constexpr int kKeys = 128;                         // keys per tile = UMMA M
-constexpr int kN = 256;                            // (queries x heads) per CTA = UMMA N
-constexpr int kStages = 3;
-constexpr uint32_t kQBytes = 2 * kN * 128;         // 65536: 2 chunks of [256 rows x 128 B]
 constexpr uint32_t kKStageBytes = 2 * kKeys * 128; // 32768
-constexpr uint32_t kOffK = kQBytes;
-constexpr uint32_t kOffW = kOffK + kStages * kKStageBytes;  // 163840
-constexpr uint32_t kOffBar = kOffW + kN * 4;
-constexpr uint32_t kSmemBytes = kOffBar + 256 + 1024;
-constexpr int kEpilogueWarps = 8;                  // warp w: keys 32 (w & 3) .. +31 of a tile, half (w >> 2) of the CTA's queries
+constexpr int kEpilogueWarps = 8;                  // warp w: keys 32 (w & 3) .. +31 of a tile
 constexpr int kMmaWarp = 8;
 constexpr int kThreads = 416;                      // 8 reduce warps, the MMA warp, 4 producer warps
-constexpr uint32_t kTmemCols = 512;
+// kN = (queries x heads) per CTA = UMMA N.  256 is the prefill shape: one CTA per SM, the two groups of four reduce warps
+// take half of the queries of every tile each.  With few queries (decode) the columns of queries that do not exist would
+// cost as much as real ones, so the smallest of 64, 128 and 256 that holds all S1 x N1 rows is taken; the narrow shapes
+// leave room for two CTAs per SM (one starts up while the other streams keys) and their reduce groups take alternate tiles.
+template <int kN>
+struct Cfg {
+  static constexpr int kCtas = kN == 256 ? 1 : 2;  // per SM
+  static constexpr int kStages = kN == 128 ? 2 : 3;
+  static constexpr bool kByTile = kN < 256;
+  static constexpr uint32_t kQBytes = 2 * kN * 128;  // 2 chunks of [kN rows x 128 B]
+  static constexpr uint32_t kOffK = kQBytes;
+  static constexpr uint32_t kOffW = kOffK + kStages * kKStageBytes;
+  static constexpr uint32_t kOffBar = kOffW + kN * 4;
+  static constexpr uint32_t kSmemBytes = kOffBar + 256;  // no slack: the base is declared (and checked) 1024-byte aligned
+  static constexpr uint32_t kTmemCols = 2 * kN;          // two accumulators
+  static_assert(kCtas * (kSmemBytes + 1024) <= 233472, "shared memory per SM");
+};
 }  // namespace itc
 
-template <bool kBF16, int N1>
-__global__ void __launch_bounds__(itc::kThreads, 1)
+template <bool kBF16, int N1, int kN>
+__global__ void __launch_bounds__(itc::kThreads, itc::Cfg<kN>::kCtas)
     indexer_scores_tc_kernel(const __grid_constant__ IndexerParams p, const __grid_constant__ CUtensorMap kmap, const int use_tma) {
   using namespace itc;
+  using C = Cfg<kN>;
+  constexpr int kStages = C::kStages;
   constexpr int QB = kN / N1;  // queries per CTA
   using T = typename std::conditional<kBF16, __nv_bfloat16, __half>::type;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sQ = smem_u32(smem);
-  const uint32_t sK = sQ + kOffK;
-  float* sW = reinterpret_cast<float*>(smem + kOffW);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kOffBar);
+  if (sQ & 1023u) {  // the swizzled operand tiles need the alignment; same in every CTA of the launch
+    if (threadIdx.x == 0) atomicCAS(p.status, kStatusOk, kStatusBadLayout);
+    return;
+  }
+  const uint32_t sK = sQ + C::kOffK;
+  float* sW = reinterpret_cast<float*>(smem + C::kOffW);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::kOffBar);
   uint64_t* k_full = bars;          // [3] count 1 + 32768 transaction bytes (TMA) or count 128 (cp.async producers)
   uint64_t* k_empty = bars + 3;     // [3] count 1 (commit)
   uint64_t* acc_full = bars + 6;    // [2] count 1 (commit)
-  uint64_t* acc_empty = bars + 8;   // [2] count 256
+  uint64_t* acc_empty = bars + 8;   // [2] count 256 (kByTile: the 128 threads of the group that reads it)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
   int* start_status = reinterpret_cast<int*>(bars + 11);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // Work unit = (chunk of tiles_per_cta key tiles, batch entry, block of queries).  First chunks come first: the last ones
+  // are empty for the shorter sequences of a ragged batch.
   const int nqb = (p.S1 + QB - 1) / QB;
-  const int b = blockIdx.x / nqb;
-  const int qb = nqb - 1 - (blockIdx.x - b * nqb);  // late (long) query blocks first
+  const int chunk = blockIdx.x / (p.B * nqb), unit = blockIdx.x - chunk * (p.B * nqb);
+  const int b = unit / nqb;
+  const int qb = nqb - 1 - (unit - b * nqb);  // late (long) query blocks first
   const int q0 = qb * QB;
 
   if (tid == 0) *start_status = *reinterpret_cast<volatile int*>(p.status);
@@ -91,15 +113,23 @@ __global__ void __launch_bounds__(itc::kThreads, 1)
     const int s1 = q0 + i;
     if (s1 < p.S1) { const int l = indexer_limit(p, b, s1, &ak); max_lim = l > max_lim ? l : max_lim; }
   }
-  const int ntiles_mma = (max_lim + kKeys - 1) / kKeys;
-  const int ntiles_all = p.fill_masked ? (p.S2 + kKeys - 1) / kKeys : ntiles_mma;
+  // this CTA's key tiles: [tile0, tile0 + ntiles_mma) are scored, those up to tile0 + ntiles_all only filled with -inf
+  const int tile0 = chunk * p.tiles_per_cta;
+  const int tiles_scored = (max_lim + kKeys - 1) / kKeys, tiles_total = p.fill_masked ? (p.S2 + kKeys - 1) / kKeys : tiles_scored;
+  const int ntiles_mma = max(0, min(tiles_scored - tile0, p.tiles_per_cta));
+  const int ntiles_all = max(0, min(tiles_total - tile0, p.tiles_per_cta));
+  if (p.limits && chunk == 0 && tid < QB && q0 + tid < p.S1) {
+    int dummy;
+    p.limits[static_cast<int64_t>(b) * p.S1 + q0 + tid] = indexer_limit(p, b, q0 + tid, &dummy);
+  }
+  if (ntiles_all == 0) return;
 
   if (tid == 0) {
     for (int i = 0; i < kStages; ++i) { mbar_init(&k_full[i], use_tma ? 1 : 128); mbar_init(&k_empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], kEpilogueWarps * 32); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], C::kByTile ? 128 : kEpilogueWarps * 32); }
     mbar_init_fence();
   }
-  if (warp == kMmaWarp) { tmem_alloc(tmem_slot, kTmemCols); tmem_relinquish(); }
+  if (warp == kMmaWarp) { tmem_alloc(tmem_slot, C::kTmemCols); tmem_relinquish(); }
   {  // Q rows (query, head) -> B operand rows; weights
     const T* qbase = reinterpret_cast<const T*>(p.q) + (static_cast<int64_t>(b) * p.S1 + q0) * N1 * kD;
     for (int u = tid; u < kN * 16; u += kThreads) {
@@ -113,10 +143,6 @@ __global__ void __launch_bounds__(itc::kThreads, 1)
       sW[r] = (q0 + r / N1 < p.S1) ? p.w[(static_cast<int64_t>(b) * p.S1 + q0) * N1 + r] : 0.f;
     cp_async_wait<0>();
     fence_proxy_async_smem();
-  }
-  if (p.limits && tid < QB && q0 + tid < p.S1) {
-    int dummy;
-    p.limits[static_cast<int64_t>(b) * p.S1 + q0 + tid] = indexer_limit(p, b, q0 + tid, &dummy);
   }
   tc_fence_before();
   __syncthreads();
@@ -143,15 +169,15 @@ __global__ void __launch_bounds__(itc::kThreads, 1)
             // a table entry that is padding (< 0) or beyond the pool gives a row coordinate outside the tensor: zeros
             const int R = p.box_rows;
             for (int j = 0; j < kKeys / R; ++j) {
-              const int key0 = it * kKeys + j * R, lb = key0 / p.block_size;
+              const int key0 = (tile0 + it) * kKeys + j * R, lb = key0 / p.block_size;
               const int phys = lb < p.max_blocks ? __ldg(p.block_table + static_cast<int64_t>(b) * p.max_blocks + lb) : -1;
               const int y = (phys >= 0 && phys < p.num_blocks) ? phys * p.block_size + key0 % p.block_size : -R;
               tma_load_2d(stage + j * R * 128, &kmap, full, 0, y);
               tma_load_2d(stage + kKeys * 128 + j * R * 128, &kmap, full, 64, y);
             }
           } else {
-            tma_load_2d(stage, &kmap, full, 0, b * p.S2 + it * kKeys);
-            tma_load_2d(stage + kKeys * 128, &kmap, full, 64, b * p.S2 + it * kKeys);
+            tma_load_2d(stage, &kmap, full, 0, b * p.S2 + (tile0 + it) * kKeys);
+            tma_load_2d(stage + kKeys * 128, &kmap, full, 64, b * p.S2 + (tile0 + it) * kKeys);
           }
         }
       }
@@ -164,7 +190,7 @@ __global__ void __launch_bounds__(itc::kThreads, 1)
       for (int j = 0; j < 16; ++j) {
         const int u = pt + 128 * j;
         const int r = u >> 4, unit = u & 15;
-        const int key = it * kKeys + r;
+        const int key = (tile0 + it) * kKeys + r;
         bool v = key < ak;
         int64_t row = key;
         if (p.block_table) {  // logical key -> row of the paged cache; padding entries of the table are not read
@@ -213,27 +239,28 @@ __global__ void __launch_bounds__(itc::kThreads, 1)
     }
   } else {
     // ================================ reduce over heads + store ====================================
-    // thread = (key, half of the CTA's queries): the accumulator row of its key, the columns of its queries
+    // thread = key: the accumulator row of its key, the columns of its queries -- of half of the CTA's queries in every tile,
+    // or (kByTile) of all of them in every other tile
     const int q4 = warp & 3, half = warp >> 2;
     const int krow = q4 * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(q4 * 32) << 16;
-    constexpr int QH = QB / 2;  // queries per thread
+    constexpr int QH = C::kByTile ? QB : QB / 2;  // queries per thread
+    const int qfirst = C::kByTile ? 0 : half * QH;
     int lim[QH];
 #pragma unroll
     for (int i = 0; i < QH; ++i) {
       int dummy;
-      const int qi = half * QH + i;
-      lim[i] = (q0 + qi < p.S1) ? indexer_limit(p, b, q0 + qi, &dummy) : 0;
+      lim[i] = (q0 + qfirst + i < p.S1) ? indexer_limit(p, b, q0 + qfirst + i, &dummy) : 0;
     }
-    float* out = p.scores + (static_cast<int64_t>(b) * p.S1 + q0 + half * QH) * p.S2;
-    for (int it = 0; it < ntiles_all; ++it) {
-      const int key = it * kKeys + krow;
+    float* out = p.scores + (static_cast<int64_t>(b) * p.S1 + q0 + qfirst) * p.S2;
+    for (int it = C::kByTile ? half : 0; it < ntiles_all; it += C::kByTile ? 2 : 1) {
+      const int key = (tile0 + it) * kKeys + krow;
       if (it < ntiles_mma) {
         const int a = it & 1;
         if (!mbar_wait(&acc_full[a], (it >> 1) & 1, p.status)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t tacc = tmem_base + a * kN + half * (kN / 2) + lane_base;
-        const float4* w4 = reinterpret_cast<const float4*>(sW + half * (kN / 2));  // weights of this half, 4 per (broadcast) load
+        const uint32_t tacc = tmem_base + a * kN + qfirst * N1 + lane_base;
+        const float4* w4 = reinterpret_cast<const float4*>(sW + qfirst * N1);  // weights of these queries, 4 per (broadcast) load
         if constexpr (N1 >= 32) {
 #pragma unroll
           for (int i = 0; i < QH; ++i) {
@@ -252,12 +279,12 @@ __global__ void __launch_bounds__(itc::kThreads, 1)
                 s1 = fmaf(w.w, fmaxf(__uint_as_float(v[4 * j + 3]), 0.f), s1);
               }
             }
-            if (q0 + half * QH + i < p.S1 && key < p.S2) out[static_cast<int64_t>(i) * p.S2 + key] = key < lim[i] ? s0 + s1 : -INFINITY;
+            if (q0 + qfirst + i < p.S1 && key < p.S2) out[static_cast<int64_t>(i) * p.S2 + key] = key < lim[i] ? s0 + s1 : -INFINITY;
           }
         } else {
           constexpr int QPC = 32 / N1;  // queries per 32-column chunk
 #pragma unroll
-          for (int cc = 0; cc < kN / 64; ++cc) {
+          for (int cc = 0; cc < QH / QPC; ++cc) {
             uint32_t v[32];
             tmem_ld32(tacc + cc * 32, v);
             tmem_wait_ld();
@@ -273,7 +300,7 @@ __global__ void __launch_bounds__(itc::kThreads, 1)
                 sum = fmaf(w.w, fmaxf(__uint_as_float(v[qq * N1 + 4 * j + 3]), 0.f), sum);
               }
               const int i = cc * QPC + qq;
-              if (q0 + half * QH + i < p.S1 && key < p.S2) out[static_cast<int64_t>(i) * p.S2 + key] = key < lim[i] ? sum : -INFINITY;
+              if (q0 + qfirst + i < p.S1 && key < p.S2) out[static_cast<int64_t>(i) * p.S2 + key] = key < lim[i] ? sum : -INFINITY;
             }
           }
         }
@@ -282,14 +309,14 @@ __global__ void __launch_bounds__(itc::kThreads, 1)
       } else if (key < p.S2) {  // tile entirely beyond every limit of this CTA
 #pragma unroll
         for (int i = 0; i < QH; ++i)
-          if (q0 + half * QH + i < p.S1) out[static_cast<int64_t>(i) * p.S2 + key] = -INFINITY;
+          if (q0 + qfirst + i < p.S1) out[static_cast<int64_t>(i) * p.S2 + key] = -INFINITY;
       }
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == kMmaWarp) tmem_dealloc(tmem_base, kTmemCols);
+  if (warp == kMmaWarp) tmem_dealloc(tmem_base, C::kTmemCols);
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -346,28 +373,45 @@ bool make_k_map(const IndexerParams& p, bool bf16, CUtensorMap* map) {
 }
 }  // namespace
 
-template <bool kBF16, int N1>
-static int launch_indexer_tc_n1(const IndexerParams& p_in, cudaStream_t stream) {
+template <bool kBF16, int N1, int kN>
+static int launch_indexer_tc_shape(const IndexerParams& p_in, cudaStream_t stream) {
   IndexerParams p = p_in;
   // rows per TMA box of a paged cache: the largest power of two (8..128) that divides the block size
   p.box_rows = 0;
   if (p.block_table)
     for (int r = itc::kKeys; r >= 8; r >>= 1)
       if (p.block_size % r == 0) { p.box_rows = r; break; }
-  auto kern = indexer_scores_tc_kernel<kBF16, N1>;
+  auto kern = indexer_scores_tc_kernel<kBF16, N1, kN>;
   int dev = 0, sms = 0;
   cudaError_t e = current_device_sms(&dev, &sms);
   if (e != cudaSuccess) return static_cast<int>(e);
-  if ((e = ensure_dynamic_smem(kern, dev, static_cast<int>(itc::kSmemBytes))) != cudaSuccess) return static_cast<int>(e);
-  constexpr int QB = itc::kN / N1;
-  const int nqb = (p.S1 + QB - 1) / QB;
+  if ((e = ensure_dynamic_smem(kern, dev, static_cast<int>(itc::Cfg<kN>::kSmemBytes))) != cudaSuccess) return static_cast<int>(e);
+  constexpr int QB = kN / N1;
+  const long long units = static_cast<long long>(p.B) * ((p.S1 + QB - 1) / QB);
+  // Keys are split into chunks, one CTA each, while the CTAs are fewer than kRounds rounds of the chip (ragged lengths even
+  // out over several rounds), but a chunk keeps at least kMinTiles tiles (a CTA's start-up costs about two tiles' time).
+  constexpr int kRounds = kN == 256 ? 2 : 4, kMinTiles = 8;
+  const int tiles = (p.S2 + itc::kKeys - 1) / itc::kKeys;
+  long long chunks = (static_cast<long long>(kRounds) * sms * itc::Cfg<kN>::kCtas + units - 1) / units;
+  if (chunks > tiles / kMinTiles) chunks = tiles / kMinTiles;
+  if (chunks < 1) chunks = 1;
+  p.tiles_per_cta = static_cast<int>((tiles + chunks - 1) / chunks);
+  chunks = (tiles + p.tiles_per_cta - 1) / p.tiles_per_cta;
   alignas(64) CUtensorMap kmap;
   memset(&kmap, 0, sizeof(kmap));
   // DSA_INDEXER_NO_TMA=1 in the environment forces the cp.async producers (used by the tests to cover that path)
   const char* no_tma = getenv("DSA_INDEXER_NO_TMA");
   const int use_tma = (!(no_tma && no_tma[0] == '1') && make_k_map(p, kBF16, &kmap)) ? 1 : 0;
-  kern<<<p.B * nqb, itc::kThreads, itc::kSmemBytes, stream>>>(p, kmap, use_tma);
+  kern<<<static_cast<unsigned>(units * chunks), itc::kThreads, itc::Cfg<kN>::kSmemBytes, stream>>>(p, kmap, use_tma);
   return static_cast<int>(cudaGetLastError());
+}
+
+template <bool kBF16, int N1>
+static int launch_indexer_tc_n1(const IndexerParams& p, cudaStream_t stream) {
+  const int rows = p.S1 < 256 ? p.S1 * N1 : 256;   // (queries x heads) of a batch entry, as far as it matters here
+  if (rows <= 64) return launch_indexer_tc_shape<kBF16, N1, 64>(p, stream);
+  if (rows <= 128) return launch_indexer_tc_shape<kBF16, N1, 128>(p, stream);
+  return launch_indexer_tc_shape<kBF16, N1, 256>(p, stream);
 }
 
 int launch_indexer_scores_tc(const IndexerParams& p, bool bf16, cudaStream_t stream) {
