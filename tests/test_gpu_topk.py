@@ -133,3 +133,36 @@ def test_rows_longer_than_shared_memory_are_streamed(rows, n, k):
         want = np.sort(ref_i[r][ref_i[r] >= 0])
         got = sets[r][sets[r] >= 0]
         assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("rows,n,top_k", [(3, 1, 1), (5, 31, 31), (2, 4096, 2048), (200, 2049, 2048), (150, 5003, 512), (7, 49152, 2048),
+                                          (3, 60001, 1000), (149, 8192, 128), (2, 20000, 8192), (160, 9000, 4096)])
+def test_bucket_select_is_exact(rows, n, top_k):
+    """Both thread counts, kept and streamed rows, odd lengths, limits, masked entries, ties inside a bucket, rows that are handed
+    to the radix select (crowded, constant, infinite): index arrays and values equal the oracle's exactly."""
+    import tilelang_ascend_b200 as dsa
+    rng = np.random.default_rng(n + top_k)
+    x = rng.standard_normal((rows, n)).astype(np.float32)
+    x[1 % rows] = np.round(x[1 % rows], 2)                       # ties, a few dozen to a value
+    x[2 % rows] = np.round(x[2 % rows] * 4) / 4                  # crowded: radix select
+    if rows > 4:
+        x[3], x[4, n // 2] = 1.5, np.inf                          # constant; infinite range
+    if rows > 6:
+        x[5, ::3] = -np.inf                                       # entries that are no candidates
+        x[6, 1:] *= np.float32(1e-3)                              # one outlier stretches the range
+        x[6, 0] = 3e4
+    x[0, ::5] *= np.float32(-0.0)                                 # zeros of both signs tie
+    lim = rng.integers(0, n + 1, size=rows).astype(np.int32)
+    lim[: (rows + 1) // 2] = n
+    for limits in (None, lim):
+        got, val = dsa.topk_select_raw(torch.from_numpy(x).cuda(), top_k, None if limits is None else torch.from_numpy(limits).cuda(), return_values=True)
+        check_status()
+        ref, ref_val = orc.topk_select(x, top_k, limits, return_values=True)
+        assert np.array_equal(got.cpu().numpy(), ref)
+        assert np.array_equal(val.cpu().numpy(), ref_val)
+    if n > 8:   # rows that do not start on 16 bytes
+        wide = torch.zeros((rows, n + 1), device="cuda")
+        wide[:, :n] = torch.from_numpy(x).cuda()
+        got = dsa.topk_select_raw(wide[:, :n], top_k).cpu().numpy()
+        assert np.array_equal(got, orc.topk_select(x, top_k))
+    check_status()
