@@ -262,6 +262,23 @@ int dsa_v4_build_indices(const int32_t* cu_seqlens_q, const int32_t* seqused_kv,
                          int32_t ori_win_left, int32_t cmp_table_len, int32_t cmp_block_size, int32_t cmp_ratio, int32_t scenario,
                          int32_t K, void* stream);
 
+/* The same lists joined for dsa_v4_attention: rows [T, ori_win_left + 1 + K] int32 (K left out in scenario 1), first the window,
+ * then the compressed keys with bit 30 set; row numbers outside their pool of ori_pool_rows / cmp_pool_rows (at most 2^30) rows
+ * become -1. */
+int dsa_v4_build_joined_indices(const int32_t* cu_seqlens_q, const int32_t* seqused_kv, const int32_t* ori_block_table,
+                                const int32_t* cmp_block_table, const int32_t* cmp_sparse_indices, int32_t* rows,
+                                int32_t ori_pool_rows, int32_t cmp_pool_rows, int32_t B, int32_t T, int32_t S, int32_t tnd,
+                                int32_t ori_table_len, int32_t ori_block_size, int32_t ori_win_left, int32_t cmp_table_len,
+                                int32_t cmp_block_size, int32_t cmp_ratio, int32_t scenario, int32_t K, void* stream);
+
+/* sparse_flash_mla in one pass: one softmax over a token's joined list and the sinks.  q [T, H, 512], ori_kv [ori_pool_rows, 512],
+ * cmp_kv [cmp_pool_rows, 512] (NULL when no row has bit 30), rows [T, width] from dsa_v4_build_joined_indices (width <= 8192),
+ * sinks [H] fp32 or NULL, out [T, H, 512], lse [T, H] fp32 or NULL (the sink is part of it; a token without keys gets out = 0 and
+ * lse = its sink).  nsplit and workspace as in dsa_sparse_mla_fwd_splitkv (B = 1, S = T, DV = 512). */
+int dsa_v4_attention(const void* q, const void* ori_kv, const void* cmp_kv, const int32_t* rows, const float* sinks, void* out,
+                     float* lse, int32_t T, int32_t H, int32_t width, int32_t ori_pool_rows, int32_t cmp_pool_rows,
+                     float sm_scale, int32_t dtype, int32_t nsplit, void* workspace, size_t workspace_bytes, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,4 +1,6 @@
 """DeepSeek-V4 sparse_flash_mla front door (window + compressed tokens + sinks) on the GPU against the oracle."""
+import importlib
+
 import numpy as np
 import pytest
 import torch
@@ -85,3 +87,38 @@ def test_sink_combine_single_partial_without_sink_is_identity():
     lse = torch.randn((5, 8), generator=g).cuda()
     o2, l2 = dsa.sink_combine_raw(out, lse, None, None, None, 8)
     assert torch.equal(o2, out) and torch.allclose(l2, lse, rtol=1e-6, atol=1e-6)
+
+
+@pytest.mark.parametrize("H,win,K,T", [(64, 127, 512, 3), (64, 0, 64, 200), (100, 63, 96, 9), (160, 127, 0, 5), (16, 127, 512, 40)])
+def test_joined_lists_match_two_passes(H, win, K, T, monkeypatch):
+    """One pass over the window and the compressed keys against the two-pass route it replaces: short and long calls (shares of a
+    split unit and whole units), several head blocks, tokens without any key, a sink far above and far below the scores, table
+    entries outside the pools.  The two routes round at different places: each is within 2^-8 of the exact row (bf16), so the
+    relative 2-norm of their difference is below 2^-7."""
+    import tilelang_ascend_b200 as dsa
+    mod = importlib.import_module("tilelang_ascend_b200.sparse_flash_mla")   # (the package re-exports the function by that name)
+    g = torch.Generator().manual_seed(H + K)
+    n_kv, ratio = 4000, 4
+    q = torch.randn((T, H, 512), generator=g).to(torch.bfloat16).cuda()
+    pool = torch.randn((32, 128, 1, 512), generator=g).to(torch.bfloat16).cuda()
+    cpool = torch.randn((70, 16, 1, 512), generator=g).to(torch.bfloat16).cuda()
+    bt = torch.randperm(32, generator=g).to(torch.int32)[None]
+    cbt = torch.randperm(70, generator=g).to(torch.int32)[None]
+    cbt[0, 3], cbt[0, 5] = -1, 70            # padding / beyond the pool: those keys take no part
+    sinks = torch.randn((H,), generator=g)
+    sinks[0], sinks[1] = 300.0, -300.0
+    kw = dict(ori_kv=pool, ori_block_table=bt.cuda(), cu_seqlens_q=torch.tensor([0, T], dtype=torch.int32).cuda(), sinks=sinks.cuda(),
+              seqused_kv=torch.tensor([n_kv if T < 100 else T - 2], dtype=torch.int32).cuda(), softmax_scale=512 ** -0.5, ori_win_left=win,
+              return_softmax_lse=True)
+    if K:
+        ci = torch.randint(0, n_kv // ratio, (T, 1, K), generator=g).sort(dim=-1).values.to(torch.int32)
+        ci[0] = -1
+        kw.update(cmp_kv=cpool, cmp_block_table=cbt.cuda(), cmp_ratio=ratio, cmp_sparse_indices=ci.cuda())
+    out, lse = dsa.sparse_flash_mla(q, **kw)
+    monkeypatch.setattr(mod, "_JOINED_MAX_KEYS", 0)
+    ref, ref_lse = dsa.sparse_flash_mla(q, **kw)
+    check_status()
+    assert torch.isfinite(lse).all() and torch.isfinite(out.float()).all()
+    assert ((out.float() - ref.float()).norm() / ref.float().norm()).item() < 2 ** -7
+    # the parts' log-sum-exps are fp32 sums of at most 640 bf16-weighted terms; merged with fast logarithms
+    assert (lse - ref_lse).abs().max().item() < 2e-3

@@ -34,6 +34,9 @@ bool block_sparse_logits_supported(const BlockSparseLogitsParams& p);
 bool block_sparse_logits_tc_supported(const BlockSparseLogitsParams& p);
 int launch_block_sparse_logits_tc(const BlockSparseLogitsParams& p, bool bf16, cudaStream_t stream);
 int launch_block_sparse_logits(const BlockSparseLogitsParams& p, bool bf16, cudaStream_t stream);
+int launch_v4_build_joined_indices(const int32_t* cu_q, const int32_t* seqused_kv, const int32_t* ori_bt, const int32_t* cmp_bt, const int32_t* cmp_idx,
+                                   int32_t* rows, int ori_pool_rows, int cmp_pool_rows, int B, int T, int S, int tnd, int ori_table_len, int ori_bs,
+                                   int win_left, int cmp_table_len, int cmp_bs, int ratio, int scenario, int K, cudaStream_t stream);
 int launch_bounded_wait_selftest(int* status, long long budget_cycles, int* gave_up, cudaStream_t stream);
 bool sparse_mla_bwd_tc_supported(const FwdParams& p);
 size_t sparse_mla_bwd_tc_bytes_per_query(int H, int topk);
@@ -110,6 +113,7 @@ int fill_fwd_params(dsa::FwdParams* p, const void* q, const void* kv, const int3
   p->block_table = block_table; p->block_size = block_size; p->max_blocks = max_blocks;
   p->scale_log2 = sm_scale * 1.4426950408889634f;
   p->nsplit = 1; p->part_out = nullptr; p->part_lse = nullptr; p->kv_rope = nullptr; p->split_queries = 0;
+  p->kv2 = nullptr; p->kv2_rows = 0; p->sinks = nullptr;
 #ifdef DSA_TRACE
   p->trace = g_trace;
 #endif
@@ -462,6 +466,50 @@ int dsa_v4_build_indices(const int32_t* cu_seqlens_q, const int32_t* seqused_kv,
                                          ori_table_len, ori_block_size, ori_win_left, cmp_table_len, cmp_block_size, cmp_ratio, scenario, K,
                                          static_cast<cudaStream_t>(stream));
   return err ? fail_cuda("v4_build_indices launch", err) : 0;
+}
+
+int dsa_v4_attention(const void* q, const void* ori_kv, const void* cmp_kv, const int32_t* rows, const float* sinks, void* out, float* lse, int32_t T,
+                     int32_t H, int32_t width, int32_t ori_pool_rows, int32_t cmp_pool_rows, float sm_scale, int32_t dtype, int32_t nsplit,
+                     void* workspace, size_t workspace_bytes, void* stream) {
+  if (cmp_pool_rows < 0 || (cmp_pool_rows > 0 && !cmp_kv)) return fail("null tensor pointer");
+  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(ori_kv) | reinterpret_cast<uintptr_t>(cmp_kv) | reinterpret_cast<uintptr_t>(out)) & 15u)
+    return fail("q, key pools and out must be 16-byte aligned");
+  dsa::FwdParams p;
+  if (fill_fwd_params(&p, q, ori_kv, rows, out, lse, 1, T, ori_pool_rows, H, 512, 512, width, sm_scale, 0, 0, dtype, nullptr, nullptr, nullptr, nullptr, 0, 0))
+    return 1;
+  p.kv2 = cmp_kv ? cmp_kv : ori_kv;
+  p.kv2_rows = cmp_kv ? cmp_pool_rows : 0;
+  p.sinks = sinks;
+  if (!dsa::sparse_mla_fwd_pair_supported(p)) return fail("lists of at most 8192 rows over pools of at most 2^30 rows");
+  if (nsplit < 1 || nsplit > 64) return fail("nsplit must be in [1, 64]");
+  if (nsplit > 1) {
+    const size_t need = dsa_sparse_mla_fwd_splitkv_workspace_bytes(1, T, H, 512, nsplit);
+    if (!workspace || workspace_bytes < need) return fail("workspace too small (see dsa_sparse_mla_fwd_splitkv_workspace_bytes)");
+    if (reinterpret_cast<uintptr_t>(workspace) & 15u) return fail("workspace must be 16-byte aligned");
+    p.nsplit = nsplit;
+    p.part_out = static_cast<float*>(workspace);
+    p.part_lse = p.part_out + static_cast<size_t>(nsplit) * T * H * 512;
+  }
+  int err = dsa::launch_sparse_mla_fwd_pair_combined(p, dtype == DSA_DTYPE_BF16, static_cast<cudaStream_t>(stream));
+  return err ? fail_cuda("v4_attention launch", err) : 0;
+}
+
+int dsa_v4_build_joined_indices(const int32_t* cu_seqlens_q, const int32_t* seqused_kv, const int32_t* ori_block_table, const int32_t* cmp_block_table,
+                                const int32_t* cmp_sparse_indices, int32_t* rows, int32_t ori_pool_rows, int32_t cmp_pool_rows, int32_t B, int32_t T,
+                                int32_t S, int32_t tnd, int32_t ori_table_len, int32_t ori_block_size, int32_t ori_win_left, int32_t cmp_table_len,
+                                int32_t cmp_block_size, int32_t cmp_ratio, int32_t scenario, int32_t K, void* stream) {
+  if (!seqused_kv || !ori_block_table || !rows) return fail("null tensor pointer");
+  if (B <= 0 || T <= 0 || ori_table_len <= 0 || ori_block_size <= 0 || ori_win_left < 0) return fail("B, T, table length and block size must be positive");
+  if (tnd ? !cu_seqlens_q : (S <= 0 || T != B * S)) return fail("packed tokens need cu_seqlens_q; otherwise T must equal B * S");
+  if (scenario < 1 || scenario > 3) return fail("scenario must be 1 (window only), 2 (all compressed tokens) or 3 (selected compressed tokens)");
+  if (scenario != 1 && (!cmp_block_table || cmp_table_len <= 0 || cmp_block_size <= 0 || cmp_ratio <= 0 || K <= 0))
+    return fail("compressed-token scenarios need the compressed block table, a positive ratio and K");
+  if (scenario == 3 && !cmp_sparse_indices) return fail("scenario 3 needs cmp_sparse_indices");
+  if (ori_pool_rows <= 0 || ori_pool_rows > dsa::kPool2Bit || cmp_pool_rows < 0 || cmp_pool_rows > dsa::kPool2Bit) return fail("pools of at most 2^30 rows");
+  int err = dsa::launch_v4_build_joined_indices(cu_seqlens_q, seqused_kv, ori_block_table, cmp_block_table, cmp_sparse_indices, rows, ori_pool_rows,
+                                                cmp_pool_rows, B, T, S, tnd, ori_table_len, ori_block_size, ori_win_left, cmp_table_len, cmp_block_size,
+                                                cmp_ratio, scenario, K, static_cast<cudaStream_t>(stream));
+  return err ? fail_cuda("v4_build_joined_indices launch", err) : 0;
 }
 
 }  // extern "C"

@@ -4,6 +4,9 @@
 
 namespace dsa {
 
+// Marks a row number of the second key pool in an index list over two pools (FwdParams::kv2).
+constexpr int kPool2Bit = 1 << 30;
+
 // Sparse MLA forward.  All tensors contiguous row-major.
 //   q        [B, S, H, D]            bf16 / fp16
 //   kv       [B, S_kv, 1, D]         (or [num_blocks, block_size, 1, D] when block_table != null)
@@ -39,6 +42,12 @@ struct FwdParams {
   // latent part) and kv_rope rows of D - DV values (the rope part), both addressed by the same row number -- the layout of
   // the dense MLA decode kernels' KV / K_pe tensors, which are then used in place instead of being concatenated first.
   const void* kv_rope;
+  // Keys from two pools (SM-pair kernel, D = DV = 512 only): when kv2 is set, an index with bit kPool2Bit set is row
+  // (index without the bit) of kv2 [kv2_rows, DV], any other one row index of kv [S_kv, DV].  No causal rule, lengths or table.
+  const void* kv2;
+  int kv2_rows;
+  // Attention sinks [H] (nullable): a logit per head that joins the softmax denominator without a value row.
+  const float* sinks;
 #ifdef DSA_TRACE
   long long* trace;            // development builds only: clock samples of cluster 0, [2 CTAs][16 events][64 tiles]
 #endif

@@ -11,6 +11,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "params.h"
+
 namespace dsa {
 
 template <typename T>
@@ -66,8 +68,12 @@ struct V4IndexParams {
   const int32_t* ori_bt;      // [B, ori_table_len]
   const int32_t* cmp_bt;      // [B, cmp_table_len] or null
   const int32_t* cmp_idx;     // [T, K] or null
-  int32_t* ori_rows;          // [T, win_left + 1]
-  int32_t* cmp_rows;          // [T, K] or null
+  int32_t* ori_rows;          // token t's window at ori_rows + t * ori_stride, win_left + 1 entries
+  int32_t* cmp_rows;          // token t's compressed keys at cmp_rows + t * cmp_stride, K entries; or null
+  int64_t ori_stride, cmp_stride;
+  // One joined list per token (two-pool form): compressed rows carry cmp_flag, rows outside their pool become -1 (they could
+  // run into the flag); separate lists have cmp_flag 0 and unlimited pools.
+  int cmp_flag, ori_pool_rows, cmp_pool_rows;
   int B, T, S, tnd;           // tnd: tokens are packed (sequence found from cu_q); else token = b * S + s
   int ori_table_len, ori_bs, win_left;
   int cmp_table_len, cmp_bs, ratio, scenario, K;
@@ -95,7 +101,8 @@ __global__ void __launch_bounds__(128) v4_build_indices_kernel(const V4IndexPara
     const int w = pos - p.win_left + i;
     int row = -1;
     if (exists && w >= 0) row = p.ori_bt[static_cast<int64_t>(b) * p.ori_table_len + w / p.ori_bs] * p.ori_bs + w % p.ori_bs;
-    p.ori_rows[static_cast<int64_t>(t) * W + i] = row;
+    if (row >= p.ori_pool_rows) row = -1;
+    p.ori_rows[static_cast<int64_t>(t) * p.ori_stride + i] = row;
   }
   if (p.scenario == 1 || !p.cmp_rows) return;
   const int threshold = exists ? (pos + 1) / p.ratio : 0;
@@ -118,15 +125,27 @@ __global__ void __launch_bounds__(128) v4_build_indices_kernel(const V4IndexPara
     }
     int row = -1;
     if (c >= 0) row = p.cmp_bt[static_cast<int64_t>(b) * p.cmp_table_len + c / p.cmp_bs] * p.cmp_bs + c % p.cmp_bs;
-    p.cmp_rows[static_cast<int64_t>(t) * p.K + i] = row;
+    if (row >= p.cmp_pool_rows) row = -1;
+    p.cmp_rows[static_cast<int64_t>(t) * p.cmp_stride + i] = row < 0 ? row : row | p.cmp_flag;
   }
 }
 
 int launch_v4_build_indices(const int32_t* cu_q, const int32_t* seqused_kv, const int32_t* ori_bt, const int32_t* cmp_bt, const int32_t* cmp_idx,
                             int32_t* ori_rows, int32_t* cmp_rows, int B, int T, int S, int tnd, int ori_table_len, int ori_bs, int win_left,
                             int cmp_table_len, int cmp_bs, int ratio, int scenario, int K, cudaStream_t stream) {
-  V4IndexParams p{cu_q, seqused_kv, ori_bt, cmp_bt, cmp_idx, ori_rows, cmp_rows, B, T, S, tnd, ori_table_len, ori_bs, win_left,
-                  cmp_table_len, cmp_bs, ratio, scenario, K};
+  V4IndexParams p{cu_q, seqused_kv, ori_bt, cmp_bt, cmp_idx, ori_rows, cmp_rows, win_left + 1, K, 0, 0x7fffffff, 0x7fffffff, B, T, S, tnd,
+                  ori_table_len, ori_bs, win_left, cmp_table_len, cmp_bs, ratio, scenario, K};
+  v4_build_indices_kernel<<<static_cast<unsigned>(T), 128, 0, stream>>>(p);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// The same lists joined, rows [T, win_left + 1 + K]: the window, then the compressed keys marked with kPool2Bit.
+int launch_v4_build_joined_indices(const int32_t* cu_q, const int32_t* seqused_kv, const int32_t* ori_bt, const int32_t* cmp_bt, const int32_t* cmp_idx,
+                                   int32_t* rows, int ori_pool_rows, int cmp_pool_rows, int B, int T, int S, int tnd, int ori_table_len, int ori_bs,
+                                   int win_left, int cmp_table_len, int cmp_bs, int ratio, int scenario, int K, cudaStream_t stream) {
+  const int W = win_left + 1, width = W + (scenario == 1 ? 0 : K);
+  V4IndexParams p{cu_q, seqused_kv, ori_bt, cmp_bt, cmp_idx, rows, scenario == 1 ? nullptr : rows + W, width, width, kPool2Bit, ori_pool_rows,
+                  cmp_pool_rows, B, T, S, tnd, ori_table_len, ori_bs, win_left, cmp_table_len, cmp_bs, ratio, scenario, K};
   v4_build_indices_kernel<<<static_cast<unsigned>(T), 128, 0, stream>>>(p);
   return static_cast<int>(cudaGetLastError());
 }

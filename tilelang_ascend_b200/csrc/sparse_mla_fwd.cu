@@ -733,13 +733,16 @@ __global__ void __launch_bounds__(256) sparse_mla_fwd_generic_kernel(const FwdPa
 // -------------------------------------------------------------------------------------------------
 // split-KV combine: out = sum_s w_s part_out[s],  w_s = exp(lse_s - lse),  lse = log sum_s exp(lse_s)
 // -------------------------------------------------------------------------------------------------
+// (an attention sink of the row's head, sinks [H] or null, joins the denominator like a share without a value row)
 template <typename T>
 __global__ void __launch_bounds__(128) sparse_mla_fwd_combine_kernel(const float* __restrict__ part_out, const float* __restrict__ part_lse,
-                                                                     T* __restrict__ out, float* __restrict__ lse, int64_t rows, int nsplit, int dv) {
+                                                                     T* __restrict__ out, float* __restrict__ lse, int64_t rows, int nsplit, int dv,
+                                                                     const float* __restrict__ sinks, int H) {
   const int64_t row = blockIdx.x;
-  float m = -INFINITY;
+  const float sk = sinks ? sinks[row % H] : -INFINITY;
+  float m = sk;
   for (int s = 0; s < nsplit; ++s) m = fmaxf(m, part_lse[s * rows + row]);
-  float wsum = 0.f;
+  float wsum = (m == -INFINITY) ? 0.f : expf(sk - m);
   for (int s = 0; s < nsplit; ++s) wsum += (m == -INFINITY) ? 0.f : expf(part_lse[s * rows + row] - m);
   for (int c = threadIdx.x * 4; c < dv; c += blockDim.x * 4) {
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -773,10 +776,10 @@ static int launch_combine(const FwdParams& p, bool bf16, cudaStream_t stream) {
   const int64_t rows = ((p.split_queries > 0 && p.split_queries < all) ? p.split_queries : all) * p.H;
   if (bf16)
     sparse_mla_fwd_combine_kernel<__nv_bfloat16><<<static_cast<unsigned>(rows), 128, 0, stream>>>(p.part_out, p.part_lse, reinterpret_cast<__nv_bfloat16*>(p.out),
-                                                                                                p.lse, rows, p.nsplit, p.DV);
+                                                                                                p.lse, rows, p.nsplit, p.DV, p.sinks, p.H);
   else
     sparse_mla_fwd_combine_kernel<__half><<<static_cast<unsigned>(rows), 128, 0, stream>>>(p.part_out, p.part_lse, reinterpret_cast<__half*>(p.out), p.lse,
-                                                                                         rows, p.nsplit, p.DV);
+                                                                                         rows, p.nsplit, p.DV, p.sinks, p.H);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -815,10 +818,10 @@ int launch_sparse_mla_fwd_tc(const FwdParams& p, bool bf16, cudaStream_t stream)
   const int64_t rows = static_cast<int64_t>(p.B) * p.S * p.H;
   if (bf16)
     sparse_mla_fwd_combine_kernel<__nv_bfloat16><<<static_cast<unsigned>(rows), 128, 0, stream>>>(p.part_out, p.part_lse, reinterpret_cast<__nv_bfloat16*>(p.out),
-                                                                                                p.lse, rows, p.nsplit, p.DV);
+                                                                                                p.lse, rows, p.nsplit, p.DV, p.sinks, p.H);
   else
     sparse_mla_fwd_combine_kernel<__half><<<static_cast<unsigned>(rows), 128, 0, stream>>>(p.part_out, p.part_lse, reinterpret_cast<__half*>(p.out), p.lse,
-                                                                                         rows, p.nsplit, p.DV);
+                                                                                         rows, p.nsplit, p.DV, p.sinks, p.H);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -25,6 +25,8 @@
 // half.  Issuing warps stay converged -- all lanes walk the loops and waits, one elected lane issues through predicated
 // instructions.  In the odd CTA lane 0 of the same four warps forwards "my gather landed" / "my softmax warps are past the
 // scores" / "my half of the swap landed" / "my P is written" to the even CTA.
+// Rows without rope dims (D = 512) can come from two pools, and an attention sink per head can join the softmax: V4's window
+// and compressed keys are then one unit, one Q load and one output instead of two of each and a pass that merges them.
 // Barriers the issuers wait for live in the even CTA and count arrivals from both CTAs; completions (tcgen05.commit) are
 // broadcast to the same barrier in both CTAs.  Every wait is bounded; a wait that gives up records status 1 and all roles
 // fall through to the teardown.
@@ -186,6 +188,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pr::kThreads, 1) spa
 #else
   auto tr = [&](int, int) {};
 #endif
+  // Does index `idx` of a unit's list take part?  (Keys from two pools: inside its pool; see FwdParams::kv2.)
+  auto takes_part = [&](const RowCtx& ctx, int idx) {
+    if constexpr (!kRope) {
+      if (p.kv2) return idx >= 0 && (idx & (kPool2Bit - 1)) < ((idx & kPool2Bit) ? p.kv2_rows : p.S_kv);
+    }
+    return index_valid(ctx, idx);
+  };
   auto bar = [&](int slot) { return bars + slot; };
   auto bar_addr = [&](int slot) { return sBars + static_cast<uint32_t>(slot) * 8u; };
 
@@ -370,13 +379,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pr::kThreads, 1) spa
       } else if (nvt == 0) {  // no key takes part, or the query does not exist (beyond q_len_b): out = 0, lse = -inf
         if (h < p.H) {
           for (int j = 0; j < 16; ++j) reinterpret_cast<uint4*>(orow)[j] = make_uint4(0, 0, 0, 0);
-          if (lse_writer && p.lse) p.lse[static_cast<int64_t>(bt) * p.H + h] = -INFINITY;
+          if (lse_writer && p.lse) p.lse[static_cast<int64_t>(bt) * p.H + h] = (!kRope && p.sinks) ? p.sinks[h] : -INFINITY;
         }
       } else {
         // the last P V of the item is complete (same barrier and argument as for the rescale above)
         if (ok) ok = __all_sync(0xffffffffu, mbar_wait(bar(kBarPFree + ((g - 1) & 1)), ((g - 1) >> 1) & 1, p.status));
         tc_fence_after();
-        const float inv_l = 1.f / l;
+        float inv_l, lse_v;
+        if (!kRope && p.sinks && shares == 1) {
+          // the head's sink joins the denominator, relative to the larger of the reference maximum and the sink itself (the
+          // shares of a split unit leave it to the combine step, which sees all of them)
+          const float sk = (h < p.H ? p.sinks[h] : -INFINITY) * 1.4426950408889634f;
+          const float m_all = fmaxf(m_used, sk), f = exp2f(m_used - m_all);
+          const float den = l * f + exp2f(sk - m_all);
+          inv_l = f / den;
+          lse_v = m_all * 0.6931471805599453f + logf(den);
+        } else {
+          inv_l = 1.f / l;
+          lse_v = m_used * 0.6931471805599453f + logf(l);
+        }
         uint32_t v[32];
 #pragma unroll 1
         for (int cc = 0; cc < 4; ++cc) {
@@ -424,7 +445,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pr::kThreads, 1) spa
           }
         }
         if (ok && lse_writer && h < p.H) {
-          const float lse_v = m_used * 0.6931471805599453f + logf(l);
           if (shares > 1) p.part_lse[prow_index] = lse_v;
           else if (p.lse) p.lse[static_cast<int64_t>(bt) * p.H + h] = lse_v;
         }
@@ -473,8 +493,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pr::kThreads, 1) spa
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
           const int tile = t0 + 4 * u;
-          const uint32_t lo = __ballot_sync(0xffffffffu, ctx.active && index_valid(ctx, i0[u]));
-          const uint32_t hi = __ballot_sync(0xffffffffu, ctx.active && index_valid(ctx, i1[u]));
+          const uint32_t lo = __ballot_sync(0xffffffffu, ctx.active && takes_part(ctx, i0[u]));
+          const uint32_t hi = __ballot_sync(0xffffffffu, ctx.active && takes_part(ctx, i1[u]));
           if (lane == 0 && tile < ntiles) masks[qp * kMaxTiles + tile] = (static_cast<unsigned long long>(hi) << 32) | lo;
         }
       }
@@ -560,7 +580,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pr::kThreads, 1) spa
       };
       // row number inside kv, -1 for a key that does not take part: it is fetched with a source size of zero, which fills
       // the destination with zeros
-      auto row_of = [&](int idx) { return index_valid(ctx, idx) ? static_cast<int>(kv_row(p, ctx.b, idx)) : -1; };
+      auto row_of = [&](int idx) {
+        if (!takes_part(ctx, idx)) return -1;
+        if constexpr (!kRope) {
+          if (p.kv2) return idx;   // already a row number (of the pool that its bit names)
+        }
+        return static_cast<int>(kv_row(p, ctx.b, idx));
+      };
       int idx_next = load_idx(0);
       int row_next = row_of(idx_next);
       idx_next = load_idx(1);
@@ -580,8 +606,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pr::kThreads, 1) spa
           const uint32_t dst = stage + sw128_offset(pw * 8 + kl, lane & 7);
           const uint32_t nbytes = row < 0 ? 0u : 16u;
           {
-            const size_t r0 = static_cast<size_t>(row < 0 ? 0 : row);
-            const uint8_t* src = kv_bytes + r0 * row_stride + (lane & 7) * 16;
+            size_t r0 = static_cast<size_t>(row < 0 ? 0 : row);
+            const uint8_t* base = kv_bytes;
+            if constexpr (!kRope) {
+              if (p.kv2 && row >= kPool2Bit) {
+                base = reinterpret_cast<const uint8_t*>(p.kv2);
+                r0 -= kPool2Bit;
+              }
+            }
+            const uint8_t* src = base + r0 * row_stride + (lane & 7) * 16;
 #pragma unroll
             for (int c = 0; c < 8; ++c) cp_async16(dst + c * kChunk, src + c * 128, nbytes);
             if (kRope) cp_async16(dst + 8 * kChunk, last_base + r0 * last_stride + (lane & 7) * 16, nbytes);
@@ -900,6 +933,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pr::kThreads, 1) spa
 // host side
 // -------------------------------------------------------------------------------------------------
 bool sparse_mla_fwd_pair_supported(const FwdParams& p) {
+  if (p.kv2 && (p.D != pr::kDV || p.S_kv > kPool2Bit || p.kv2_rows > kPool2Bit)) return false;
   // (row numbers inside kv are kept in 32 bits by the gather warps)
   return (p.D == pr::kD || p.D == pr::kDV) && p.DV == pr::kDV && p.topk <= pr::kMaxTiles * pr::kBK &&
          static_cast<long long>(p.B) * p.S_kv <= 0x7fffffffLL;
