@@ -86,6 +86,13 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t smem_dst, const void* src
                : "memory");
 }
 
+// Adds four fp32 values (given as bits) to 16-byte aligned global memory.
+__device__ __forceinline__ void red_add_v4(float* dst, const uint4& v) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(__uint_as_float(v.x)), "f"(__uint_as_float(v.y)),
+               "f"(__uint_as_float(v.z)), "f"(__uint_as_float(v.w))
+               : "memory");
+}
+
 // 16 gathered rows (one per entry of rows[], -1 = zero fill) x kChunks chunks of 64 dims starting at chunk `chunk0` of
 // the row, into the K-major / 128-byte-swizzle chunk images of a stage: chunk c at stage + c * kChunkBytes, key
 // 16 pw + kk is row 16 pw + kk of every chunk.  Lane = (chunk within a group of four, 16-byte unit).
@@ -543,8 +550,8 @@ constexpr uint32_t kOffQ = kStages * kPairBytes;                // 98304
 constexpr uint32_t kOffDO = kOffQ + kOperandBytes;              // 147456
 constexpr uint32_t kOffBar = kOffDO + kOperandBytes;            // 196608
 constexpr uint32_t kOffMask = kOffBar + 128;
-constexpr uint32_t kOffXpose = kOffMask + kMaxTiles * 8;        // per epilogue warp: [32 keys x 16 dims] fp32 + 32 row numbers
-constexpr uint32_t kXposeBytes = 32 * 64 + 128;
+constexpr uint32_t kOffXpose = kOffMask + kMaxTiles * 8;        // per epilogue warp: [32 keys x 32 dims] fp32
+constexpr uint32_t kXposeBytes = 32 * 128;
 constexpr int kEpilogueWarps = 8;                               // warp w: tensor-memory lanes 32 (w & 3) .., columns 96 (w >> 2) .. + 95
 constexpr int kLoadWarp = 8, kIssueWarp = 9;
 constexpr int kThreadsDkv = 320;
@@ -680,9 +687,7 @@ __global__ void __launch_bounds__(bwdtc::dkv::kThreadsDkv, 1) sparse_mla_bwd_dkv
       mbar_arrive(b_ready);
     }
     const int32_t* idx_row = p.indices + static_cast<int64_t>(bt) * p.topk;
-    uint8_t* xbuf_ptr = smem + kOffXpose + warp * kXposeBytes;
-    const uint32_t xbuf = smem_u32(xbuf_ptr);
-    int* xrows = reinterpret_cast<int*>(xbuf_ptr + 32 * 64);
+    const uint32_t xbuf = sBase + kOffXpose + warp * kXposeBytes;
     int g = 0;
     for (int tp = 0; run && ok && tp < npairs; ++tp) {
       const unsigned long long m0 = smask[2 * tp], m1 = smask[2 * tp + 1];
@@ -690,9 +695,8 @@ __global__ void __launch_bounds__(bwdtc::dkv::kThreadsDkv, 1) sparse_mla_bwd_dkv
       const int ab = g & 1;
       const bool valid = ((r < 64 ? m0 >> r : m1 >> (r - 64)) & 1ull) != 0ull;
       const int idx = valid ? __ldg(idx_row + tp * 128 + r) : 0;
-      // row number inside dKV of this thread's key (-1: takes no part), shared with the warp for the transposed atomics
-      __syncwarp();
-      xrows[lane] = valid ? static_cast<int>(kv_row_of(p, b, idx)) : -1;
+      // row number inside dKV of this thread's key, -1: takes no part
+      const int my_row = valid ? static_cast<int>(kv_row_of(p, b, idx)) : -1;
       if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[ab], (g >> 1) & 1, p.status))) { ok = false; break; }
       tc_fence_after();
       // this thread's 96 columns leave tensor memory at once, so that the accumulator goes back to the MMA issuer before
@@ -704,31 +708,25 @@ __global__ void __launch_bounds__(bwdtc::dkv::kThreadsDkv, 1) sparse_mla_bwd_dkv
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_free[ab]);
-      int rows4[4];
+      float* dst = bp.d_kv + part * kDimsPerCta + half * 96 + (lane & 7) * 4;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) rows4[i] = xrows[i * 8 + (lane >> 2)];
-#pragma unroll
-      for (int cc = 0; cc < 6; ++cc) {  // chunks of 16 columns
-        // The warp holds [32 keys x 16 dims] with one key per lane.  Through shared memory (16-byte units XOR-swizzled by the
-        // row, conflict-free both ways) it is turned so that 4 consecutive lanes cover the 64 contiguous bytes of ONE key:
-        // an atomic instruction then touches 16 full sectors instead of 32 half-used ones.
+      for (int cc = 0; cc < 3; ++cc) {  // chunks of 32 columns
+        // The warp holds [32 keys x 32 dims] with one key per lane.  Through shared memory (16-byte units XOR-swizzled by the
+        // row, conflict-free both ways) it is turned so that eight consecutive lanes cover 128 contiguous bytes of ONE key: an
+        // add then touches four whole lines.  (This kernel is bound by the LSU pipe, 79 % busy, and the requests it sends to
+        // L2, 75 %; with 16 columns at a time an add touched half of eight lines: 978 -> 917 us per 1184 queries of 128 heads.)
         __syncwarp();
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          st_shared_v4(xbuf + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4), v[16 * cc + 4 * j], v[16 * cc + 4 * j + 1], v[16 * cc + 4 * j + 2],
-                       v[16 * cc + 4 * j + 3]);
+        for (int j = 0; j < 8; ++j)
+          st_shared_v4(xbuf + sw128_offset(lane, j), v[32 * cc + 4 * j], v[32 * cc + 4 * j + 1], v[32 * cc + 4 * j + 2], v[32 * cc + 4 * j + 3]);
         __syncwarp();
-        float4 val[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int key = i * 8 + (lane >> 2);
-          val[i] = *reinterpret_cast<const float4*>(xbuf_ptr + key * 64 + (((lane & 3) ^ ((key >> 1) & 3)) << 4));
+        for (int i = 0; i < 8; ++i) {
+          const int key = i * 4 + (lane >> 3);
+          const uint4 val = ld_shared_v4(xbuf + sw128_offset(key, lane & 7));
+          const int row = __shfl_sync(0xffffffffu, my_row, key);
+          if (row >= 0) red_add_v4(dst + static_cast<int64_t>(row) * kD + cc * 32, val);
         }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (rows4[i] >= 0)
-            atomicAdd(reinterpret_cast<float4*>(bp.d_kv + static_cast<int64_t>(rows4[i]) * kD + part * kDimsPerCta + half * 96 + cc * 16) + (lane & 3),
-                      val[i]);
       }
       ++g;
     }
