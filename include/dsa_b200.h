@@ -187,6 +187,15 @@ int dsa_sparse_mla_fwd_two_part(const void* q, const void* kv_latent, const void
                                 int32_t q_start, int32_t causal, int32_t dtype, const int32_t* q_start_b, const int32_t* kv_len_b,
                                 const int32_t* q_len_b, const int32_t* block_table, int32_t block_size, int32_t max_blocks, int32_t nsplit,
                                 void* workspace, size_t workspace_bytes, void* stream);
+
+/* The same with the queries in two parts as well: q_latent [B, S, H, DV] and q_rope [B, S, H, D - DV], 16-byte aligned (the Q / Q_pe
+ * tensors of the decode kernels, used in place instead of being concatenated by the caller). */
+int dsa_sparse_mla_fwd_two_part_q(const void* q_latent, const void* q_rope, const void* kv_latent, const void* kv_rope,
+                                  const int32_t* indices, void* out, float* lse, int32_t B, int32_t S, int32_t S_kv, int32_t H,
+                                  int32_t D, int32_t DV, int32_t topk, float sm_scale, int32_t q_start, int32_t causal,
+                                  int32_t dtype, const int32_t* q_start_b, const int32_t* kv_len_b, const int32_t* q_len_b,
+                                  const int32_t* block_table, int32_t block_size, int32_t max_blocks, int32_t nsplit,
+                                  void* workspace, size_t workspace_bytes, void* stream);
 int dsa_sparse_mla_fwd_splitkv_nsplit(int32_t B, int32_t S, int32_t H, int32_t topk);
 size_t dsa_sparse_mla_fwd_splitkv_workspace_bytes(int32_t B, int32_t S, int32_t H, int32_t DV, int32_t nsplit);
 int dsa_sparse_mla_fwd_splitkv(const void* q, const void* kv, const int32_t* indices, void* out, float* lse, int32_t B,

@@ -150,3 +150,25 @@ def test_argument_rules():
     with pytest.raises(ValueError, match="shapes"):
         dsa.mla_decode(1, 64, 1, 128, 512, 64)(q, torch.zeros((1, 64, 64), dtype=H16, device=DEV),
                                                torch.zeros((1, 64, 1, 512), dtype=H16, device=DEV), torch.zeros((1, 64, 1, 64), dtype=H16, device=DEV))
+
+
+@pytest.mark.parametrize("H,B,N,nsplit,dtype", [(1, 3, 70, 1, torch.bfloat16), (64, 5, 300, 3, torch.float16), (100, 80, 129, 1, torch.bfloat16),
+                                                (128, 2, 2048, None, torch.float16), (200, 40, 64, 1, torch.bfloat16)])
+def test_queries_in_two_parts_equal_concatenated_queries(H, B, N, nsplit, dtype):
+    """The kernel that reads latent and rope dims of the queries from two tensors: bit-equal to the call on rows of 576, with
+    ragged head blocks, several units per cluster and shares of a unit; parts that do not start on 16 bytes are concatenated."""
+    g = torch.Generator().manual_seed(H)
+    q, qr = torch.randn((B, 1, H, 512), generator=g).to(DEV, dtype), torch.randn((B, 1, H, 64), generator=g).to(DEV, dtype)
+    kv, kr = torch.randn((B, N, 1, 512), generator=g).to(DEV, dtype), torch.randn((B, N, 1, 64), generator=g).to(DEV, dtype)
+    idx = torch.arange(N, dtype=torch.int32, device=DEV).expand(B, 1, 1, N).contiguous()
+    kw = dict(sm_scale=576 ** -0.5, q_start=0, causal=False, dv=512, nsplit=nsplit, kv_rope=kr)
+    ref, ref_lse = dsa.sparse_mla_fwd_raw(torch.cat((q, qr), dim=-1), kv, idx, **kw)
+    out, lse = dsa.sparse_mla_fwd_raw(q, kv, idx, q_rope=qr, **kw)
+    check_status()
+    assert torch.equal(out, ref) and torch.equal(lse, ref_lse)
+    odd = torch.empty(q.numel() + 1, dtype=dtype, device=DEV)[1:].view(q.shape).copy_(q)
+    got = dsa.mla_decode(B, H, 1, N, 512, 64)(odd[:, 0], qr[:, 0], kv, kr)
+    check_status()
+    assert torch.equal(got, ref[:, 0]) if nsplit is None else torch.isfinite(got).all()
+    with pytest.raises(ValueError):
+        dsa.sparse_mla_fwd_raw(q, kv, idx, q_rope=qr[..., :32].contiguous(), **kw)

@@ -48,6 +48,9 @@ SIGNATURES = {
     "dsa_sparse_mla_fwd_two_part": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32,
                                               c_int32, c_int32, c_int32, c_float, c_int32, c_int32, c_int32, c_void_p, c_void_p, c_void_p,
                                               c_void_p, c_int32, c_int32, c_int32, c_void_p, c_size_t, c_void_p]),
+    "dsa_sparse_mla_fwd_two_part_q": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32,
+                                              c_int32, c_int32, c_int32, c_float, c_int32, c_int32, c_int32, c_void_p, c_void_p, c_void_p,
+                                              c_void_p, c_int32, c_int32, c_int32, c_void_p, c_size_t, c_void_p]),
     "dsa_sparse_mla_fwd_splitkv_nsplit": (c_int32, [c_int32, c_int32, c_int32, c_int32]),
     "dsa_sparse_mla_fwd_splitkv_workspace_bytes": (c_size_t, [c_int32, c_int32, c_int32, c_int32, c_int32]),
     "dsa_sparse_mla_fwd_splitkv": (c_int32, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_int32, c_int32, c_int32,

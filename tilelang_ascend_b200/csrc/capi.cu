@@ -113,7 +113,7 @@ int fill_fwd_params(dsa::FwdParams* p, const void* q, const void* kv, const int3
   p->block_table = block_table; p->block_size = block_size; p->max_blocks = max_blocks;
   p->scale_log2 = sm_scale * 1.4426950408889634f;
   p->nsplit = 1; p->part_out = nullptr; p->part_lse = nullptr; p->kv_rope = nullptr; p->split_queries = 0;
-  p->kv2 = nullptr; p->kv2_rows = 0; p->sinks = nullptr;
+  p->q_rope = nullptr; p->kv2 = nullptr; p->kv2_rows = 0; p->sinks = nullptr;
 #ifdef DSA_TRACE
   p->trace = g_trace;
 #endif
@@ -288,11 +288,11 @@ int dsa_sparse_mla_fwd(const void* q, const void* kv, const int32_t* indices, vo
   return err ? fail_cuda("sparse_mla_fwd launch", err) : 0;
 }
 
-int dsa_sparse_mla_fwd_two_part(const void* q, const void* kv_latent, const void* kv_rope, const int32_t* indices, void* out, float* lse,
-                                int32_t B, int32_t S, int32_t S_kv, int32_t H, int32_t D, int32_t DV, int32_t topk, float sm_scale,
-                                int32_t q_start, int32_t causal, int32_t dtype, const int32_t* q_start_b, const int32_t* kv_len_b,
-                                const int32_t* q_len_b, const int32_t* block_table, int32_t block_size, int32_t max_blocks, int32_t nsplit,
-                                void* workspace, size_t workspace_bytes, void* stream) {
+static int fwd_two_part_impl(const void* q, const void* q_rope, const void* kv_latent, const void* kv_rope, const int32_t* indices, void* out, float* lse,
+                             int32_t B, int32_t S, int32_t S_kv, int32_t H, int32_t D, int32_t DV, int32_t topk, float sm_scale,
+                             int32_t q_start, int32_t causal, int32_t dtype, const int32_t* q_start_b, const int32_t* kv_len_b,
+                             const int32_t* q_len_b, const int32_t* block_table, int32_t block_size, int32_t max_blocks, int32_t nsplit,
+                             void* workspace, size_t workspace_bytes, void* stream) {
   if (!kv_rope) return fail("null tensor pointer");
   if (D != 576 || DV != 512) return fail("key rows in two parts need D = 576 and DV = 512");
   if ((reinterpret_cast<uintptr_t>(kv_latent) | reinterpret_cast<uintptr_t>(kv_rope)) & 15u) return fail("key tensors must be 16-byte aligned");
@@ -302,6 +302,7 @@ int dsa_sparse_mla_fwd_two_part(const void* q, const void* kv_latent, const void
     return 1;
   if (!dsa::sparse_mla_fwd_pair_supported(p)) return fail("key rows in two parts need topk <= 8192");
   p.kv_rope = kv_rope;
+  p.q_rope = q_rope;
   if (nsplit < 1 || nsplit > 64) return fail("nsplit must be in [1, 64]");
   if (nsplit > 1) {
     const size_t need = dsa_sparse_mla_fwd_splitkv_workspace_bytes(B, S, H, DV, nsplit);
@@ -313,6 +314,26 @@ int dsa_sparse_mla_fwd_two_part(const void* q, const void* kv_latent, const void
   }
   int err = dsa::launch_sparse_mla_fwd_pair_combined(p, dtype == DSA_DTYPE_BF16, static_cast<cudaStream_t>(stream));
   return err ? fail_cuda("sparse_mla_fwd_two_part launch", err) : 0;
+}
+
+int dsa_sparse_mla_fwd_two_part(const void* q, const void* kv_latent, const void* kv_rope, const int32_t* indices, void* out, float* lse,
+                                int32_t B, int32_t S, int32_t S_kv, int32_t H, int32_t D, int32_t DV, int32_t topk, float sm_scale,
+                                int32_t q_start, int32_t causal, int32_t dtype, const int32_t* q_start_b, const int32_t* kv_len_b,
+                                const int32_t* q_len_b, const int32_t* block_table, int32_t block_size, int32_t max_blocks, int32_t nsplit,
+                                void* workspace, size_t workspace_bytes, void* stream) {
+  return fwd_two_part_impl(q, nullptr, kv_latent, kv_rope, indices, out, lse, B, S, S_kv, H, D, DV, topk, sm_scale, q_start, causal, dtype, q_start_b,
+                           kv_len_b, q_len_b, block_table, block_size, max_blocks, nsplit, workspace, workspace_bytes, stream);
+}
+
+int dsa_sparse_mla_fwd_two_part_q(const void* q_latent, const void* q_rope, const void* kv_latent, const void* kv_rope, const int32_t* indices,
+                                  void* out, float* lse, int32_t B, int32_t S, int32_t S_kv, int32_t H, int32_t D, int32_t DV, int32_t topk,
+                                  float sm_scale, int32_t q_start, int32_t causal, int32_t dtype, const int32_t* q_start_b, const int32_t* kv_len_b,
+                                  const int32_t* q_len_b, const int32_t* block_table, int32_t block_size, int32_t max_blocks, int32_t nsplit,
+                                  void* workspace, size_t workspace_bytes, void* stream) {
+  if (!q_rope) return fail("null tensor pointer");
+  if ((reinterpret_cast<uintptr_t>(q_latent) | reinterpret_cast<uintptr_t>(q_rope)) & 15u) return fail("query tensors must be 16-byte aligned");
+  return fwd_two_part_impl(q_latent, q_rope, kv_latent, kv_rope, indices, out, lse, B, S, S_kv, H, D, DV, topk, sm_scale, q_start, causal, dtype,
+                           q_start_b, kv_len_b, q_len_b, block_table, block_size, max_blocks, nsplit, workspace, workspace_bytes, stream);
 }
 
 int dsa_sparse_mla_fwd_splitkv_nsplit(int32_t B, int32_t S, int32_t H, int32_t topk) {

@@ -42,6 +42,8 @@ struct FwdParams {
   // latent part) and kv_rope rows of D - DV values (the rope part), both addressed by the same row number -- the layout of
   // the dense MLA decode kernels' KV / K_pe tensors, which are then used in place instead of being concatenated first.
   const void* kv_rope;
+  // The same for queries: when q_rope is set, q holds [B, S, H, DV] and q_rope [B, S, H, D - DV].
+  const void* q_rope;
   // Keys from two pools (SM-pair kernel, D = DV = 512 only): when kv2 is set, an index with bit kPool2Bit set is row
   // (index without the bit) of kv2 [kv2_rows, DV], any other one row index of kv [S_kv, DV].  No causal rule, lengths or table.
   const void* kv2;

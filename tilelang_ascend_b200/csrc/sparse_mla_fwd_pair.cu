@@ -126,7 +126,8 @@ __device__ __forceinline__ void st_async_v4_b32(uint32_t cluster_addr, uint32_t 
                : "memory");
 }
 
-template <bool kBF16, bool kRope>
+// kQTwo: the queries come in two parts (FwdParams::q_rope).  A template parameter: deciding it at run time cost the prefill 3 %.
+template <bool kBF16, bool kRope, bool kQTwo>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pr::kThreads, 1) sparse_mla_fwd_pair_kernel(const FwdParams p) {
   using namespace pr;
   constexpr int kRowBytes = kRope ? kD * 2 : kDV * 2;
@@ -198,17 +199,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pr::kThreads, 1) spa
   auto bar = [&](int slot) { return bars + slot; };
   auto bar_addr = [&](int slot) { return sBars + static_cast<uint32_t>(slot) * 8u; };
 
-  // First Q row (head 64 r of the unit's head block) of work unit `u` and the number of this CTA's 64 rows that exist
-  // (nullptr / 0 when the unit does not exist).  The 64 rows are contiguous in q: 64 x kRowBytes bytes.
-  auto q_rows_of = [&](int u, int* nrows) -> const uint8_t* {
+  // Number of the first Q row (head 64 r of the unit's head block) of work unit `u` in q, and the number of this CTA's 64
+  // rows that exist (0 when the unit does not exist).  The 64 rows are consecutive.
+  auto q_rows_of = [&](int u, int* nrows) -> int64_t {
     *nrows = 0;
-    if (u < 0) return nullptr;
+    if (u < 0) return 0;
     int sh_unused, ns_unused;
     const int it_item = item_and_share(u, &sh_unused, &ns_unused);
     const int nbt = it_item / head_blocks, nh0 = (it_item - nbt * head_blocks) * kM + static_cast<int>(rank) * kHeads;
-    if (nh0 >= p.H) return nullptr;
+    if (nh0 >= p.H) return 0;
     *nrows = p.H - nh0 < kHeads ? p.H - nh0 : kHeads;
-    return reinterpret_cast<const uint8_t*>(p.q) + (static_cast<int64_t>(nbt) * p.H + nh0) * kRowBytes;
+    return static_cast<int64_t>(nbt) * p.H + nh0;
   };
 
   // ---- setup ------------------------------------------------------------------------------------------
@@ -535,7 +536,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pr::kThreads, 1) spa
         // the item boundary the exchange warps only move them from shared memory to tensor memory.  Slot j: dims 192 j ..
         // 192 j + 191 as three chunks of [64 rows x 128 bytes] (128-byte swizzle); one instruction copies 128 bytes of four rows.
         int nrows;
-        const uint8_t* q0 = q_rows_of(unit, &nrows);
+        const int64_t qrow0 = q_rows_of(unit, &nrows);
+        // rows in one piece, or (kQTwo) in two parts like the keys' (q_rope: dims 512..)
+        constexpr int q_stride = kQTwo ? kDV * 2 : kRowBytes;
+        const uint8_t* q0 = reinterpret_cast<const uint8_t*>(p.q) + qrow0 * q_stride;
+        const uint8_t* qr0 = kQTwo ? reinterpret_cast<const uint8_t*>(p.q_rope) + qrow0 * ((kD - kDV) * 2) : nullptr;
         const int gt = tid - kFirstGatherWarp * 32;
 #pragma unroll 1
         for (int j = 0; j < 2; ++j) {
@@ -550,7 +555,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pr::kThreads, 1) spa
                 const int row = (gt >> 3) + 16 * i, unit16 = gt & 7;
                 const bool v = row < nrows;
                 cp_async16(stage + cj * kQChunk + sw128_offset(row, unit16),
-                           v ? q0 + row * kRowBytes + (3 * j + cj) * 128 + unit16 * 16 : reinterpret_cast<const uint8_t*>(p.q), v ? 16u : 0u);
+                           v ? q0 + row * q_stride + (3 * j + cj) * 128 + unit16 * 16 : reinterpret_cast<const uint8_t*>(p.q), v ? 16u : 0u);
               }
             // ... and behind them half of the dims that stay in shared memory (384..), as pieces of [64 rows x 32 dims]: 64
             // bytes per row, the four 16-byte units of a row permuted by (row / 2) % 4, so that both these copies (64 bytes of
@@ -561,9 +566,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pr::kThreads, 1) spa
               for (int i = 0; i < 2; ++i) {
                 const int row = (gt >> 2) + 32 * i, u16 = gt & 3;
                 const bool v = row < nrows;
+                const int piece = kQPiecesPerSlot * j + pc;   // dims 384 + 32 piece ..: pieces 4 and 5 are the rope dims
+                const uint8_t* src = (!kQTwo || piece < 4) ? q0 + row * q_stride + 768 + piece * 64 : qr0 + row * ((kD - kDV) * 2) + (piece - 4) * 64;
                 cp_async16(stage + kQPieceOff + pc * kQPiece + row * 64 + ((u16 ^ ((row >> 1) & 3)) << 4),
-                           v ? q0 + row * kRowBytes + 768 + (kQPiecesPerSlot * j + pc) * 64 + u16 * 16 : reinterpret_cast<const uint8_t*>(p.q),
-                           v ? 16u : 0u);
+                           v ? src + u16 * 16 : reinterpret_cast<const uint8_t*>(p.q), v ? 16u : 0u);
               }
             cp_async_arrive_noinc(bar(kBarKvFull + s));
           }
@@ -944,8 +950,9 @@ int launch_sparse_mla_fwd_pair(const FwdParams& p, bool bf16, cudaStream_t strea
   cudaError_t e = current_device_sms(&dev, &sms);
   if (e != cudaSuccess) return static_cast<int>(e);
   const bool rope = p.D == pr::kD;
-  auto kern = rope ? (bf16 ? sparse_mla_fwd_pair_kernel<true, true> : sparse_mla_fwd_pair_kernel<false, true>)
-                   : (bf16 ? sparse_mla_fwd_pair_kernel<true, false> : sparse_mla_fwd_pair_kernel<false, false>);
+  auto kern = !rope ? (bf16 ? sparse_mla_fwd_pair_kernel<true, false, false> : sparse_mla_fwd_pair_kernel<false, false, false>)
+              : p.q_rope ? (bf16 ? sparse_mla_fwd_pair_kernel<true, true, true> : sparse_mla_fwd_pair_kernel<false, true, true>)
+                         : (bf16 ? sparse_mla_fwd_pair_kernel<true, true, false> : sparse_mla_fwd_pair_kernel<false, true, false>);
   if ((e = ensure_dynamic_smem(kern, dev, static_cast<int>(pr::kSmemBytes))) != cudaSuccess) return static_cast<int>(e);
   // persistent: one 2-CTA cluster per SM pair, each walking its share of the (query, head block) items
   long long clusters = sms / 2 > 0 ? sms / 2 : 1;

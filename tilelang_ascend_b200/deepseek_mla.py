@@ -15,7 +15,7 @@ import functools
 import torch
 
 from .adapter import check_inputs
-from .sparse_flash_attention import sparse_mla_fwd_raw
+from .sparse_flash_attention import queries_in_two_parts, sparse_mla_fwd_raw
 
 # the tensor-core forward walks index lists of up to this many keys; the dense decode has no other kernel to fall to
 MAX_KEYS = 8192
@@ -26,6 +26,14 @@ def _identity_indices(cache: dict, dev, batch: int, n: int) -> torch.Tensor:
     if key not in cache:
         cache[key] = torch.arange(n, dtype=torch.int32, device=dev).view(1, 1, 1, n).expand(batch, 1, 1, n).contiguous()
     return cache[key]
+
+
+def _queries(q, q_pe, key_parts: bool):
+    """([B,1,H,D], None), or the two parts ([B,1,H,dim], [B,1,H,pe]) where the kernel that reads keys in two parts can take the
+    queries that way too (no concatenated copy per call)."""
+    if key_parts and queries_in_two_parts(q, q_pe):
+        return q.unsqueeze(1), q_pe.unsqueeze(1)
+    return torch.cat((q, q_pe), dim=-1).unsqueeze(1).contiguous(), None
 
 
 def _check_keys(n: int) -> None:
@@ -54,12 +62,12 @@ class MlaDecodeKernel:
         if tuple(q.shape) != (B, H, self.dim) or tuple(q_pe.shape) != (B, H, self.pe_dim) \
                 or tuple(kv.shape) != (B, N, 1, self.dim) or tuple(k_pe.shape) != (B, N, 1, self.pe_dim):
             raise ValueError("input shapes differ from the factory arguments")
-        qq = torch.cat((q, q_pe), dim=-1).unsqueeze(1).contiguous()
+        qq, qq_pe = _queries(q, q_pe, self.dim == 512 and self.pe_dim == 64)
         idx = _identity_indices(self._idx, dev, B, self.actual)
         scale = (self.dim + self.pe_dim) ** -0.5
         if self.dim == 512 and self.pe_dim == 64:
             # kv and k_pe are read in place (rows in two parts): no concatenated copy of the cache per call
-            out, _ = sparse_mla_fwd_raw(qq, kv, idx, sm_scale=scale, q_start=0, causal=False, dv=self.dim, return_lse=False, kv_rope=k_pe)
+            out, _ = sparse_mla_fwd_raw(qq, kv, idx, sm_scale=scale, q_start=0, causal=False, dv=self.dim, return_lse=False, kv_rope=k_pe, q_rope=qq_pe)
         else:
             kk = torch.cat((kv, k_pe), dim=-1).contiguous()
             out, _ = sparse_mla_fwd_raw(qq, kk, idx, sm_scale=scale, q_start=0, causal=False, dv=self.dim, return_lse=False)
@@ -97,7 +105,7 @@ class MlaDecodePagedKernel:
         if tuple(Q.shape) != (B, H, self.dv) or tuple(Q_pe.shape) != (B, H, self.dpe) or tuple(KV.shape) != (rows, 1, self.dv) \
                 or tuple(K_pe.shape) != (rows, 1, self.dpe) or tuple(block_table.shape) != (B, nb):
             raise ValueError("input shapes differ from the factory arguments")
-        qq = torch.cat((Q, Q_pe), dim=-1).unsqueeze(1).contiguous()
+        qq, qq_pe = _queries(Q, Q_pe, self.dv == 512 and self.dpe == 64)
         if dev not in self._len:
             self._len[dev] = torch.full((B,), self.cache_seqlen, dtype=torch.int32, device=dev)
         idx = _identity_indices(self._idx, dev, B, self.cache_seqlen)
@@ -106,7 +114,7 @@ class MlaDecodePagedKernel:
         nblk = rows // self.block_size
         if self.dv == 512 and self.dpe == 64:
             # the two pools are read in place through the same block table (rows in two parts)
-            out, _ = sparse_mla_fwd_raw(qq, KV.view(nblk, self.block_size, 1, self.dv), idx, kv_rope=K_pe.view(nblk, self.block_size, 1, self.dpe),
+            out, _ = sparse_mla_fwd_raw(qq, KV.view(nblk, self.block_size, 1, self.dv), idx, kv_rope=K_pe.view(nblk, self.block_size, 1, self.dpe), q_rope=qq_pe,
                                         **common)
         else:
             pool = torch.cat((KV, K_pe), dim=-1).view(nblk, self.block_size, 1, self.dv + self.dpe)
@@ -147,12 +155,12 @@ class MlaDecodePersistentKernel:
         if tuple(Q.shape) != (B, H, self.dim) or tuple(Q_pe.shape) != (B, H, self.pe_dim) or tuple(KV.shape) != (B, N, self.dim) \
                 or tuple(K_pe.shape) != (B, N, self.pe_dim):
             raise ValueError("input shapes differ from the factory arguments")
-        qq = torch.cat((Q, Q_pe), dim=-1).unsqueeze(1).contiguous()
+        qq, qq_pe = _queries(Q, Q_pe, self.dim == 512 and self.pe_dim == 64)
         idx = _identity_indices(self._idx, dev, B, N)
         scale = (self.dim + self.pe_dim) ** -0.5
         if self.dim == 512 and self.pe_dim == 64:   # KV and K_pe read in place (rows in two parts)
             out, _ = sparse_mla_fwd_raw(qq, KV.unsqueeze(2), idx, sm_scale=scale, q_start=0, causal=False, dv=self.dim, return_lse=False,
-                                        kv_rope=K_pe.unsqueeze(2))
+                                        kv_rope=K_pe.unsqueeze(2), q_rope=qq_pe)
         else:
             kk = torch.cat((KV, K_pe), dim=-1).unsqueeze(2).contiguous()
             out, _ = sparse_mla_fwd_raw(qq, kk, idx, sm_scale=scale, q_start=0, causal=False, dv=self.dim, return_lse=False)

@@ -51,7 +51,7 @@ def _next_pow2(x: int) -> int:
 
 def sparse_mla_fwd_raw(q, kv, indices, *, sm_scale: float, q_start: int, causal: bool, dv: int, out=None,
                        return_lse: bool = True, q_start_b=None, kv_len_b=None, q_len_b=None, block_table=None,
-                       block_size: int = 0, impl: int = _lib.IMPL_AUTO, nsplit=None, kv_rope=None, split_queries: int = 0):
+                       block_size: int = 0, impl: int = _lib.IMPL_AUTO, nsplit=None, kv_rope=None, split_queries: int = 0, q_rope=None):
     """One launch of the forward through the C ABI.  q [B,S,H,D], kv [B,S_kv,1,D] (or paged blocks),
     indices [B,S,1,topk] int32.  Returns (out, lse-or-None).
 
@@ -67,11 +67,14 @@ def sparse_mla_fwd_raw(q, kv, indices, *, sm_scale: float, q_start: int, causal:
 
     ``kv_rope``: key rows in two parts -- ``kv`` then holds the dv latent values of every row ([B,S_kv,1,dv] or paged blocks)
     and ``kv_rope`` the D - dv rope values with the same leading shape (the KV / K_pe tensors of the dense MLA decode
-    kernels, used in place); D = 576, dv = 512, topk <= 8192 only."""
+    kernels, used in place); D = 576, dv = 512, topk <= 8192 only.  ``q_rope`` [B,S,H,D - dv] (with ``kv_rope`` only): the same for
+    the queries, ``q`` then being [B,S,H,dv]."""
     if kv_rope is not None:
         return _fwd_two_part(q, kv, kv_rope, indices, sm_scale=sm_scale, q_start=q_start, causal=causal, dv=dv, return_lse=return_lse,
                              q_start_b=q_start_b, kv_len_b=kv_len_b, q_len_b=q_len_b, block_table=block_table, block_size=block_size,
-                             nsplit=nsplit)
+                             nsplit=nsplit, q_rope=q_rope)
+    if q_rope is not None:
+        raise ValueError("q_rope needs kv_rope")
     opt = [t for t in (q_start_b, kv_len_b, q_len_b, block_table) if t is not None]
     dev = check_inputs([q, kv, indices] + opt, [None, q.dtype, torch.int32] + [torch.int32] * len(opt),
                        ["q", "kv", "indices"] + ["int32 side input"] * len(opt))
@@ -127,13 +130,24 @@ def sparse_mla_fwd_raw(q, kv, indices, *, sm_scale: float, q_start: int, causal:
     return out, lse
 
 
+def queries_in_two_parts(q, q_rope) -> bool:
+    """Can the kernel read these latent (512) and rope (64) parts of the queries in place?"""
+    return (q.shape[-1] == 512 and q_rope.shape[-1] == 64 and q.shape[:-1] == q_rope.shape[:-1] and q.dtype == q_rope.dtype and q.device == q_rope.device
+            and q.is_contiguous() and q_rope.is_contiguous() and q.data_ptr() % 16 == 0 and q_rope.data_ptr() % 16 == 0)
+
+
 def _fwd_two_part(q, kv, kv_rope, indices, *, sm_scale, q_start, causal, dv, return_lse, q_start_b, kv_len_b, q_len_b, block_table,
-                  block_size, nsplit):
+                  block_size, nsplit, q_rope=None):
     opt = [t for t in (q_start_b, kv_len_b, q_len_b, block_table) if t is not None]
     dev = check_inputs([q, kv, kv_rope, indices] + opt, [None, q.dtype, q.dtype, torch.int32] + [torch.int32] * len(opt),
                        ["q", "kv", "kv_rope", "indices"] + ["int32 side input"] * len(opt))
     code = dtype_code(q.dtype)
     B, S, H, D = q.shape
+    if q_rope is not None:
+        check_inputs([q, q_rope], [None, q.dtype], ["q", "q_rope"])
+        if D != dv or q_rope.shape != (B, S, H, q_rope.shape[-1]):
+            raise ValueError(f"queries in two parts need q [B,S,H,{dv}] and q_rope of equal leading shape (got {tuple(q.shape)}, {tuple(q_rope.shape)})")
+        D += q_rope.shape[-1]
     if D != 576 or dv != 512 or kv.dim() != 4 or kv_rope.dim() != 4 or kv.shape[2:] != (1, dv) or kv_rope.shape[2:] != (1, D - dv) \
             or kv.shape[:2] != kv_rope.shape[:2] or indices.shape[:3] != (B, S, 1):
         raise ValueError(f"key rows in two parts need D = 576, dv = 512, kv [...,1,512] and kv_rope [...,1,64] of equal leading shape "
@@ -156,8 +170,9 @@ def _fwd_two_part(q, kv, kv_rope, indices, *, sm_scale, q_start, causal, dv, ret
         nsplit = int(lib.dsa_sparse_mla_fwd_splitkv_nsplit(B, S, H, topk)) if nsplit is None else int(nsplit)
         nbytes = int(lib.dsa_sparse_mla_fwd_splitkv_workspace_bytes(B, S, H, dv, nsplit)) if nsplit > 1 else 0
         workspace = _split_workspace(dev, nbytes) if nsplit > 1 else None
-        _lib.check(lib.dsa_sparse_mla_fwd_two_part(
-            ptr(q), ptr(kv), ptr(kv_rope), ptr(indices), ptr(out), ptr(lse), B, S, S_kv, H, D, dv, topk, float(sm_scale), int(q_start),
+        entry, queries = (lib.dsa_sparse_mla_fwd_two_part, (ptr(q),)) if q_rope is None else (lib.dsa_sparse_mla_fwd_two_part_q, (ptr(q), ptr(q_rope)))
+        _lib.check(entry(
+            *queries, ptr(kv), ptr(kv_rope), ptr(indices), ptr(out), ptr(lse), B, S, S_kv, H, D, dv, topk, float(sm_scale), int(q_start),
             1 if causal else 0, code, ptr(q_start_b), ptr(kv_len_b), ptr(q_len_b), ptr(block_table), int(block_size), int(max_blocks),
             nsplit, ptr(workspace), nbytes, current_stream(dev)))
     return out, lse
@@ -281,12 +296,14 @@ def sparse_attn_tilelang(query, key, value, sparse_indices, scale_value, sparse_
     squeeze = query.dim() == 3
     if squeeze:
         query, query_rope, sparse_indices = query.unsqueeze(0), query_rope.unsqueeze(0), sparse_indices.unsqueeze(0)
-    q = torch.cat((query, query_rope), dim=-1).contiguous()
     # the key cache and its rope part are read in place as the two parts of a key row where the kernel can do that
     # (512 + 64 values, lists of at most 8192 keys); otherwise they are concatenated into rows of D values first
     two_part = (key.shape[-1] == 512 and key_rope.shape[-1] == 64 and sparse_indices.shape[-1] <= 8192 and key.is_contiguous()
                 and key_rope.is_contiguous())
     kv = key if two_part else torch.cat((key, key_rope), dim=-1).contiguous()
+    # ... and so are the queries and their rope part (a copy of both per call otherwise)
+    two_part_q = two_part and queries_in_two_parts(query, query_rope)
+    q = query if two_part_q else torch.cat((query, query_rope), dim=-1).contiguous()
     dev = q.device
     B, S = q.shape[0], q.shape[1]
     act_q = torch.as_tensor(actual_seq_lengths_query, dtype=torch.int32).to(dev).contiguous()
@@ -300,7 +317,8 @@ def sparse_attn_tilelang(query, key, value, sparse_indices, scale_value, sparse_
     out, lse = sparse_mla_fwd_raw(q, kv, sparse_indices.to(torch.int32).contiguous(), sm_scale=float(scale_value), q_start=0,
                                   causal=(sparse_mode == 3), dv=query.shape[-1], return_lse=return_softmax_lse,
                                   q_start_b=q_start_b, kv_len_b=act_kv, q_len_b=act_q, block_table=bt,
-                                  block_size=kv.shape[1] if bt is not None else 0, kv_rope=key_rope if two_part else None)
+                                  block_size=kv.shape[1] if bt is not None else 0, kv_rope=key_rope if two_part else None,
+                                  q_rope=query_rope if two_part_q else None)
     if squeeze:
         out = out.squeeze(0)
         lse = lse.squeeze(0) if lse is not None else None
