@@ -1,4 +1,6 @@
 """Lightning indexer on the GPU against the reference fixtures and the oracle."""
+import importlib
+
 import numpy as np
 import pytest
 import torch
@@ -327,3 +329,35 @@ def test_few_queries_over_chunks_of_keys(B, S1, N1, S2, paged, monkeypatch):
                                           block_table=perm, layout_key="PA_BSND", sparse_count=K)[0]
             assert torch.equal(got_p, dense)
         check_status()
+
+
+@pytest.mark.parametrize("where", ["cuda", "cpu"])
+def test_lengths_known_to_the_device_or_the_host(where, monkeypatch):
+    """Paged keys: launched over the table's width before the lengths are read, or over the longest length when the workspace would
+    be too large: the same indices; too long lengths raise, empty batches give -1, wherever the lengths live."""
+    import tilelang_ascend_b200 as dsa
+    mod = importlib.import_module("tilelang_ascend_b200.lightning_indexer")
+    B, S1, bs, nb = 3, 2, 16, 40
+    q, k, w = orc.make_indexer_inputs(B, S1, nb * bs, 32, 128, seed=4)
+    table = torch.randperm(B * nb, generator=torch.Generator().manual_seed(2)).to(torch.int32).view(B, nb)
+    pool = torch.empty((B * nb, bs, 1, 128), dtype=k.dtype)
+    pool[table.long().view(-1)] = k.view(B * nb, bs, 1, 128)
+    q, w, pool, table = q.cuda(), w.cuda(), pool.cuda(), table.cuda()
+
+    def call(ak, aq=(2, 2, 1)):
+        return dsa.lightning_indexer(q, pool, w, actual_seq_lengths_query=torch.tensor(aq, dtype=torch.int32, device=where),
+                                     actual_seq_lengths_key=torch.tensor(ak, dtype=torch.int32, device=where), block_table=table,
+                                     layout_key="PA_BSND", sparse_count=64)[0]
+
+    wide = call((77, 500, 0))
+    monkeypatch.setattr(mod, "_EARLY_LAUNCH_MAX_BYTES", 0)
+    exact = call((77, 500, 0))
+    monkeypatch.undo()
+    check_status()
+    assert torch.equal(wide, exact) and wide.shape == (B, S1, 1, 64) and bool((wide[2] == -1).all())
+    for ak, aq in (((0, 0, 0), (2, 2, 1)), ((77, 500, 3), (0, 0, 0))):
+        none = call(ak, aq)
+        assert none.shape == (B * S1, 1, 64) and bool((none == -1).all())
+    with pytest.raises(ValueError):
+        call((77, nb * bs + 1, 3))
+    check_status()
