@@ -733,18 +733,19 @@ __global__ void __launch_bounds__(bwdtc::dkv::kThreadsDkv, 1) sparse_mla_bwd_dkv
         // The warp holds [32 keys x 32 dims] with one key per lane.  Through shared memory (16-byte units XOR-swizzled by the
         // row, conflict-free both ways) it is turned so that eight consecutive lanes cover 128 contiguous bytes of ONE key: an
         // add then touches four whole lines.  (This kernel is bound by the LSU pipe, 79 % busy, and the requests it sends to
-        // L2, 75 %; with 16 columns at a time an add touched half of eight lines: 978 -> 917 us per 1184 queries of 128 heads.)
+        // L2, 75 %; with 16 columns at a time an add touched half of eight lines: 978 -> 917 us per 1184 queries of 128 heads; all loads of a step before its adds: 900 us.)
         __syncwarp();
 #pragma unroll
         for (int j = 0; j < 8; ++j)
           st_shared_v4(xbuf + sw128_offset(lane, j), v[32 * cc + 4 * j], v[32 * cc + 4 * j + 1], v[32 * cc + 4 * j + 2], v[32 * cc + 4 * j + 3]);
         __syncwarp();
+        uint4 val[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) val[i] = ld_shared_v4(xbuf + sw128_offset(i * 4 + (lane >> 3), lane & 7));
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const int key = i * 4 + (lane >> 3);
-          const uint4 val = ld_shared_v4(xbuf + sw128_offset(key, lane & 7));
-          const int row = __shfl_sync(0xffffffffu, my_row, key);
-          if (row >= 0) red_add_v4(dst + static_cast<int64_t>(row) * kD + cc * 32, val);
+          const int row = __shfl_sync(0xffffffffu, my_row, i * 4 + (lane >> 3));
+          if (row >= 0) red_add_v4(dst + static_cast<int64_t>(row) * kD + cc * 32, val[i]);
         }
       }
       ++g;
