@@ -360,3 +360,45 @@ def test_split_tail_rows_are_combined_and_all_other_rows_stay_bit_equal(S, m, n,
     kernel = dsa.sparse_attention_fwd(H, 512, 64, 320, 1, return_softmax_lse=True)
     k_o, k_l = kernel(q.cuda(), kv.cuda(), idx.cuda(), split_tail=(m, n))
     assert torch.equal(k_o.cpu(), out) and torch.equal(k_l.cpu(), lse)
+
+
+@pytest.mark.parametrize("B,S,S_kv,H,D,topk,nsplit,paged,dtype", [
+    (1, 1, 1, 1, 576, 1, 1, False, torch.bfloat16), (1, 3, 33, 64, 512, 33, 1, False, torch.float16), (2, 150, 700, 64, 576, 512, 1, False, torch.bfloat16),
+    (3, 5, 2100, 17, 576, 2048, 3, True, torch.float16), (1, 40, 4500, 32, 576, 4096, None, False, torch.bfloat16), (4, 2, 900, 64, 576, 100, 16, True, torch.bfloat16),
+    (1, 333, 64, 63, 512, 64, 1, False, torch.bfloat16), (1, 20, 5000, 64, 576, 4160, 1, False, torch.bfloat16)])
+def test_up_to_64_heads_match_the_pair_kernel(B, S, S_kv, H, D, topk, nsplit, paged, dtype, monkeypatch):
+    """The kernel for at most 64 heads against the SM-pair kernel (the last row is beyond its lists and runs the same kernel twice):
+    one to all heads, lists from one key to the longest, empty lists, several units per CTA, shares, paged keys, growing maxima (the
+    rescale).  Outputs are rounded to 16 bits once by either kernel, from P rounded to 16 bits: relative 2-norm below 2^-7."""
+    import tilelang_ascend_b200 as dsa
+    g = torch.Generator().manual_seed(H * 7 + topk)
+    q = torch.randn((B, S, H, D), generator=g).to("cuda", dtype)
+    kv = torch.randn((B, S_kv, 1, D), generator=g)
+    kv *= torch.linspace(0.3, 4.0, S_kv)[None, :, None, None]     # later keys score higher: the reference maximum keeps growing
+    kv = kv.to("cuda", dtype)
+    idx = torch.randint(-1, S_kv + 3, (B, S, 1, topk), generator=g).sort(dim=-1).values.to(torch.int32)
+    idx[0, 0] = -1                                                # no key at all
+    idx[-1, -1, 0, : topk // 2] = -1                              # leading tiles are empty
+    kw = dict(sm_scale=D ** -0.5, q_start=S_kv - S, causal=True, dv=512, nsplit=nsplit)
+    keys = kv
+    if paged:
+        bs = 20
+        nb = -(-S_kv // bs)
+        table = torch.randperm(B * nb, generator=g).to(torch.int32).view(B, nb)
+        keys = torch.zeros((B * nb, bs, 1, D), dtype=dtype, device="cuda")
+        pad = torch.zeros((B, nb * bs, 1, D), dtype=dtype, device="cuda")
+        pad[:, :S_kv] = kv
+        keys[table.long().view(-1).cuda()] = pad.view(B * nb, bs, 1, D)
+        lens = torch.tensor([S_kv - 3 * b for b in range(B)], dtype=torch.int32)
+        kw.update(block_table=table.cuda(), block_size=bs, kv_len_b=lens.cuda(), q_len_b=torch.full((B,), max(S - 1, 1), dtype=torch.int32).cuda(),
+                  q_start_b=(lens - S).cuda())
+    out, lse = dsa.sparse_mla_fwd_raw(q, keys, idx.cuda(), **kw)
+    monkeypatch.setenv("DSA_FWD_KERNEL", "pair")
+    ref, ref_lse = dsa.sparse_mla_fwd_raw(q, keys, idx.cuda(), **{**kw, "nsplit": 1})
+    check_status()
+    assert torch.equal(torch.isinf(lse), torch.isinf(ref_lse)) and torch.isfinite(out.float()).all()
+    fin = torch.isfinite(lse)
+    if fin.any():
+        assert (lse - ref_lse)[fin].abs().max().item() < 1e-3
+        assert ((out.float() - ref.float()).norm() / ref.float().norm()).item() < 2 ** -7
+    assert not bool(out[~fin].any())

@@ -826,9 +826,12 @@ int launch_sparse_mla_fwd_tc(const FwdParams& p, bool bf16, cudaStream_t stream)
 }
 
 // Number of shares that fills the GPU's cluster slots when there are fewer (query, head block) items than slots.
+bool sparse_mla_fwd_narrow_shape(int H, int topk);
+
 int sparse_mla_fwd_auto_nsplit(const FwdParams& p, int sms) {
   const long long items = static_cast<long long>(p.B) * p.S * ((p.H + tc::kM - 1) / tc::kM);
-  const long long clusters = sms / 2 > 0 ? sms / 2 : 1;
+  const long long slots = sparse_mla_fwd_narrow_shape(p.H, p.topk) ? sms : sms / 2;   // a CTA or a pair of CTAs per item
+  const long long clusters = slots > 0 ? slots : 1;
   const int ntiles = (p.topk + tc::kBK - 1) / tc::kBK;
   long long ns = clusters / (items > 0 ? items : 1);
   if (ns > 16) ns = 16;
