@@ -367,7 +367,7 @@ def test_split_tail_rows_are_combined_and_all_other_rows_stay_bit_equal(S, m, n,
     (3, 5, 2100, 17, 576, 2048, 3, True, torch.float16), (1, 40, 4500, 32, 576, 4096, None, False, torch.bfloat16), (4, 2, 900, 64, 576, 100, 16, True, torch.bfloat16),
     (1, 333, 64, 63, 512, 64, 1, False, torch.bfloat16), (1, 20, 5000, 64, 576, 4160, 1, False, torch.bfloat16)])
 def test_up_to_64_heads_match_the_pair_kernel(B, S, S_kv, H, D, topk, nsplit, paged, dtype, monkeypatch):
-    """The kernel for at most 64 heads against the SM-pair kernel (the last row is beyond its lists and runs the same kernel twice):
+    """The kernel for at most 64 heads against the SM-pair kernel (rows with lists of more than 2048 keys run that one twice):
     one to all heads, lists from one key to the longest, empty lists, several units per CTA, shares, paged keys, growing maxima (the
     rescale).  Outputs are rounded to 16 bits once by either kernel, from P rounded to 16 bits: relative 2-norm below 2^-7."""
     import tilelang_ascend_b200 as dsa
@@ -402,3 +402,16 @@ def test_up_to_64_heads_match_the_pair_kernel(B, S, S_kv, H, D, topk, nsplit, pa
         assert (lse - ref_lse)[fin].abs().max().item() < 1e-3
         assert ((out.float() - ref.float()).norm() / ref.float().norm()).item() < 2 ** -7
     assert not bool(out[~fin].any())
+
+
+def test_queries_that_start_between_sectors_take_the_pair_kernel(monkeypatch):
+    """The kernel for at most 64 heads reads queries 32 bytes at a time; a view that starts on 16 bytes only is still accepted."""
+    import tilelang_ascend_b200 as dsa
+    q, kv, idx = orc.make_sparse_mla_inputs(1, 20, 300, 64, 128, seed=2)
+    shifted = torch.empty(q.numel() + 8, dtype=q.dtype, device="cuda")[8:].view(q.shape).copy_(q)
+    kw = dict(sm_scale=576 ** -0.5, q_start=280, causal=True, dv=512, nsplit=1)
+    out, lse = dsa.sparse_mla_fwd_raw(shifted, kv.cuda(), idx.cuda(), **kw)
+    monkeypatch.setenv("DSA_FWD_KERNEL", "pair")
+    ref, ref_lse = dsa.sparse_mla_fwd_raw(q.cuda(), kv.cuda(), idx.cuda(), **kw)
+    check_status()
+    assert torch.equal(out, ref) and torch.equal(lse, ref_lse)

@@ -947,13 +947,13 @@ bool sparse_mla_fwd_pair_supported(const FwdParams& p) {
          static_cast<long long>(p.B) * p.S_kv <= 0x7fffffffLL;
 }
 
-bool sparse_mla_fwd_narrow_shape(int H, int topk);
+bool sparse_mla_fwd_narrow_supported(const FwdParams& p);
 int launch_sparse_mla_fwd_narrow(const FwdParams& p, bool bf16, cudaStream_t stream);
 
 int launch_sparse_mla_fwd_pair(const FwdParams& p, bool bf16, cudaStream_t stream) {
   // At most 64 heads: the kernel of one CTA per query (DSA_FWD_KERNEL=pair in the environment keeps this one, as a cross-check).
   const char* which = getenv("DSA_FWD_KERNEL");
-  if (sparse_mla_fwd_narrow_shape(p.H, p.topk) && !(which && which[0] == 'p')) return launch_sparse_mla_fwd_narrow(p, bf16, stream);
+  if (sparse_mla_fwd_narrow_supported(p) && !(which && which[0] == 'p')) return launch_sparse_mla_fwd_narrow(p, bf16, stream);
   int dev = 0, sms = 0;
   cudaError_t e = current_device_sms(&dev, &sms);
   if (e != cudaSuccess) return static_cast<int>(e);
