@@ -9,8 +9,9 @@
 //     (MN-major), B = P as the softmax wrote it.  The accumulator has one output dim per lane and the heads in its columns, so
 //     a rescale multiplies columns by factors that the softmax leaves in shared memory.
 // What bounds it: ~1300 clocks per tile of 32 keys, the time from a stage's refill to its release (gather ~1000, Q K^T ~2000 with
-// two in flight, softmax ~1100, P V ~600) over five (D = 512: six) stages; and ~4000 clocks at a unit's end, where the next
-// unit's Q goes to tensor memory while the ring is full.  Tiles of 32 keys rather than 64 are what gives the ring its stages.
+// two in flight, softmax ~1100, P V ~600) over five (D = 512: six) stages, with 6.6 TB/s of rows coming out of L2.  Sending Q
+// through the ring as the pair kernel does, instead of ~4000 clocks of loads at a unit's end, changed neither by more than
+// the runs differ (310 -> 305, 976 -> 976 us).  Tiles of 32 keys rather than 64 are what gives the ring its stages.
 // Measured (CUDA events, 8192 queries of 64 heads with 128 + 512 keys / 2 x 777 queries with 1024 keys): the pair kernel 1640 /
 // 485 us; one Q K^T issuer, one softmax group 1230 / 457; two issuers 1058 / 334; two softmax groups, Q in tensor memory for one
 // or two more stages, lists one unit ahead 990 / 321; Q in whole sectors, its second half requested before the rest 976 / 310.
