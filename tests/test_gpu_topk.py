@@ -136,9 +136,10 @@ def test_rows_longer_than_shared_memory_are_streamed(rows, n, k):
 
 
 @pytest.mark.parametrize("rows,n,top_k", [(3, 1, 1), (5, 31, 31), (2, 4096, 2048), (200, 2049, 2048), (150, 5003, 512), (7, 49152, 2048),
-                                          (3, 60001, 1000), (149, 8192, 128), (2, 20000, 8192), (160, 9000, 4096)])
+                                          (3, 60001, 1000), (149, 8192, 128), (2, 20000, 8192), (160, 9000, 4096),
+                                          (50, 50001, 700), (37, 49152, 2048), (1, 131072, 2048), (1, 200003, 8192)])
 def test_bucket_select_is_exact(rows, n, top_k):
-    """Both thread counts, kept and streamed rows, odd lengths, limits, masked entries, ties inside a bucket, rows that are handed
+    """Both thread counts, one CTA and clusters of 4 and 8 per row, kept and streamed rows, odd lengths, limits, masked entries, ties inside a bucket, rows that are handed
     to the radix select (crowded, constant, infinite): index arrays and values equal the oracle's exactly."""
     import tilelang_ascend_b200 as dsa
     rng = np.random.default_rng(n + top_k)

@@ -19,6 +19,7 @@
 #include <stdint.h>
 
 #include "launch_util.h"
+#include "ptx.cuh"
 
 namespace dsa {
 
@@ -353,8 +354,27 @@ __global__ void __launch_bounds__(topk::kSelectThreads, kMaxRounds <= 4 ? 4 : 1)
 // (larger key, or equal key and lower index): a handful of comparisons, no sort, no search inside the threshold's bucket.
 // Rows whose values crowd (more than kMaxPerBucket in a bucket that is needed, a range that is zero or not finite) take the
 // radix select.  4096 rows of up to 8192 -> 2048: 380 -> 112 us; 64 rows of 4096 -> 2048, whole call: 22.5 -> 15.0 us.
-// kCache: the row stays in shared memory after the first pass; longer rows are read three times (from L2).
-template <int kThreads, bool kCache, int kMaxRounds>
+// kC > 1: a cluster of kC CTAs per row, each with a contiguous slice of it (few long rows: one CTA per row leaves most SMs idle
+// and is bound by its own shared-memory atomics).  The CTAs exchange their ranges, sum the histograms bucket range by bucket
+// range into the first CTA's, and put the elements into its list; the rest is the first CTA's work.
+// kCache: the row (slice) stays in shared memory after the first pass; longer rows are read three times (from L2).
+// Shared memory of the CTA that a mapped address names.
+__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t v) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+__device__ __forceinline__ void st_cluster_u64(uint32_t addr, unsigned long long v) {
+  asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t atom_add_cluster_u32(uint32_t addr, uint32_t v) {
+  uint32_t old;
+  asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(addr), "r"(v) : "memory");
+  return old;
+}
+
+template <int kThreads, bool kCache, int kMaxRounds, int kC>
 __global__ void __launch_bounds__(kThreads, (kThreads == 512 && kMaxRounds <= 4) ? 3 : 1)
     topk_bucket_kernel(const float* __restrict__ scores, int64_t row_stride, int n_all, const int32_t* __restrict__ limits, int top_k, int kp,
                        int32_t* __restrict__ out_idx, float* __restrict__ out_val) {
@@ -367,12 +387,16 @@ __global__ void __launch_bounds__(kThreads, (kThreads == 512 && kMaxRounds <= 4)
   __shared__ float w_min[kWarps], w_max[kWarps];
   __shared__ uint32_t w_sum[kWarps], w_fullest[kWarps], w_total[kWarps];
   __shared__ int s_last;
+  __shared__ uint32_t s_fullest;
+  __shared__ float s_range[2];   // this CTA's minimum and maximum (kC > 1)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int row = blockIdx.x;
+  const int row = blockIdx.x / kC;
+  const uint32_t rank = kC > 1 ? cluster_ctarank() : 0u;
   const float* x = scores + static_cast<int64_t>(row) * row_stride;
   int n = limits ? limits[row] : n_all;
   n = n < 0 ? 0 : (n > n_all ? n_all : n);
-  const int n4 = (n + 3) >> 2;
+  const int n4 = (n + 3) >> 2, per4 = (n4 + kC - 1) / kC;
+  const int beg4 = static_cast<int>(rank) * per4, end4 = min(n4, beg4 + per4);   // this CTA's groups of four
   // (16-byte groups of the row: never past its end when its length is a multiple of four)
   const bool vec = (n_all & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
   // candidates 4 i4 .. + 3; what is not a candidate reads as -inf
@@ -395,24 +419,24 @@ __global__ void __launch_bounds__(kThreads, (kThreads == 512 && kMaxRounds <= 4)
     return v;
   };
   auto get4 = [&](int i4) -> float4 {
-    if constexpr (kCache) return reinterpret_cast<const float4*>(cache)[i4];
+    if constexpr (kCache) return reinterpret_cast<const float4*>(cache)[i4 - beg4];
     else return load4(i4);
   };
 
   // ---- range of the candidates ----
   for (int i = tid; i < kBuckets; i += kThreads) bucket[i] = 0;
   float mn = INFINITY, mx = -INFINITY;
-  for (int base = tid; base < n4; base += 4 * kThreads) {
+  for (int base = beg4 + tid; base < end4; base += 4 * kThreads) {
     float4 v[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int i4 = base + u * kThreads;
-      v[u] = i4 < n4 ? load4(i4) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+      v[u] = i4 < end4 ? load4(i4) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int i4 = base + u * kThreads;
-      if (kCache && i4 < n4) reinterpret_cast<float4*>(cache)[i4] = v[u];
+      if (kCache && i4 < end4) reinterpret_cast<float4*>(cache)[i4 - beg4] = v[u];
       mx = fmaxf(fmaxf(fmaxf(mx, v[u].x), fmaxf(v[u].y, v[u].z)), v[u].w);
       const float f[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
 #pragma unroll
@@ -434,17 +458,35 @@ __global__ void __launch_bounds__(kThreads, (kThreads == 512 && kMaxRounds <= 4)
     mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   }
+  if constexpr (kC > 1) {
+    if (tid == 0) { s_range[0] = mn; s_range[1] = mx; }
+    cluster_sync_all();
+#pragma unroll
+    for (int r = 0; r < kC; ++r) {
+      const uint32_t a = map_to_cta(smem_u32(s_range), r);
+      mn = fminf(mn, __uint_as_float(ld_cluster_u32(a)));
+      mx = fmaxf(mx, __uint_as_float(ld_cluster_u32(a + 4)));
+    }
+  }
+  // the way out of a row that the buckets do not suit (kC > 1: no CTA touches another's memory any more, the first one works alone)
+  auto radix = [&]() {
+    if constexpr (kC > 1) {
+      cluster_sync_all();
+      if (rank != 0) return;
+    }
+    __syncthreads();
+    radix_select_row<kThreads, kMaxRounds, (!kCache || kC > 1)>(smem_raw, row, scores, row_stride, n_all, limits, top_k, kp, out_idx, out_val, 1);
+  };
   const float scale = static_cast<float>(kBuckets) / (mx - mn);
   if (!(scale > 0.f && scale < 3e38f && mx - mn < 3e38f)) {  // no candidates, equal values, a range that is not finite
-    __syncthreads();
-    radix_select_row<kThreads, kMaxRounds, !kCache>(smem_raw, row, scores, row_stride, n_all, limits, top_k, kp, out_idx, out_val, 1);
+    radix();
     return;
   }
   auto bucket_of = [&](float f) { return min(static_cast<int>((mx - f) * scale), kBuckets - 1); };
 
   // ---- histogram ----
 #pragma unroll 2
-  for (int i4 = tid; i4 < n4; i4 += kThreads) {
+  for (int i4 = beg4 + tid; i4 < end4; i4 += kThreads) {
     const float4 v = get4(i4);
     const float f[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -453,48 +495,69 @@ __global__ void __launch_bounds__(kThreads, (kThreads == 512 && kMaxRounds <= 4)
   }
   __syncthreads();
 
-  // ---- starts of the buckets, the last one that is needed, the fullest one of those ----
-  uint32_t c[kPer], mine = 0;
+  const uint32_t lead_bucket = kC > 1 ? map_to_cta(smem_u32(bucket), 0) : 0u, lead_list = kC > 1 ? map_to_cta(smem_u32(list), 0) : 0u;
+  if constexpr (kC > 1) {  // every CTA sums one range of the buckets over all of them, in the first one's histogram
+    cluster_sync_all();
+    for (int b = static_cast<int>(rank) * (kBuckets / kC) + tid; b < static_cast<int>(rank + 1) * (kBuckets / kC); b += kThreads) {
+      uint32_t sum = 0;
 #pragma unroll
-  for (int j = 0; j < kPer; ++j) { c[j] = bucket[tid * kPer + j]; mine += c[j]; }
-  uint32_t incl = mine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
+      for (int r = 0; r < kC; ++r) sum += ld_cluster_u32(map_to_cta(smem_u32(bucket + b), r));
+      st_cluster_u32(lead_bucket + b * 4, sum);
+    }
+    cluster_sync_all();
   }
-  if (lane == 31) w_sum[warp] = incl;
-  __syncthreads();
-  uint32_t start = incl - mine;
-  for (int w = 0; w < warp; ++w) start += w_sum[w];
+
+  // ---- starts of the buckets, the last one that is needed, the fullest one of those ----
   const uint32_t want = static_cast<uint32_t>(top_k);
   uint32_t fullest = 0, total = 0;   // total: elements in the buckets up to the last one, fewer than top_k + kMaxPerBucket
+  if (rank == 0) {
+    uint32_t c[kPer], mine = 0;
 #pragma unroll
-  for (int j = 0; j < kPer; ++j) {
-    bucket[tid * kPer + j] = start;
-    if (start < want) {   // a bucket with places among the first top_k
-      fullest = max(fullest, c[j]);
-      total = start + c[j];
-      if (start + c[j] >= want) s_last = tid * kPer + j;   // (one thread, one bucket: where the count passes top_k)
+    for (int j = 0; j < kPer; ++j) { c[j] = bucket[tid * kPer + j]; mine += c[j]; }
+    uint32_t incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
     }
-    start += c[j];
-  }
-  fullest = __reduce_max_sync(0xffffffffu, fullest);
-  total = __reduce_max_sync(0xffffffffu, total);
-  if (lane == 0) { w_fullest[warp] = fullest; w_total[warp] = total; }
-  __syncthreads();
-  fullest = __reduce_max_sync(0xffffffffu, w_fullest[lane % kWarps]);
-  total = __reduce_max_sync(0xffffffffu, w_total[lane % kWarps]);
-  if (fullest > static_cast<uint32_t>(kMaxPerBucket)) {
+    if (lane == 31) w_sum[warp] = incl;
     __syncthreads();
-    radix_select_row<kThreads, kMaxRounds, !kCache>(smem_raw, row, scores, row_stride, n_all, limits, top_k, kp, out_idx, out_val, 1);
+    uint32_t start = incl - mine;
+    for (int w = 0; w < warp; ++w) start += w_sum[w];
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      bucket[tid * kPer + j] = start;
+      if (start < want) {   // a bucket with places among the first top_k
+        fullest = max(fullest, c[j]);
+        total = start + c[j];
+        if (start + c[j] >= want) s_last = tid * kPer + j;   // (one thread, one bucket: where the count passes top_k)
+      }
+      start += c[j];
+    }
+    fullest = __reduce_max_sync(0xffffffffu, fullest);
+    total = __reduce_max_sync(0xffffffffu, total);
+    if (lane == 0) { w_fullest[warp] = fullest; w_total[warp] = total; }
+    __syncthreads();
+    fullest = __reduce_max_sync(0xffffffffu, w_fullest[lane % kWarps]);
+    total = __reduce_max_sync(0xffffffffu, w_total[lane % kWarps]);
+    if (kC > 1 && tid == 0) s_fullest = fullest;
+  }
+  int last = 0;
+  if constexpr (kC > 1) {
+    cluster_sync_all();
+    last = static_cast<int>(ld_cluster_u32(map_to_cta(smem_u32(&s_last), 0)));
+    fullest = ld_cluster_u32(map_to_cta(smem_u32(&s_fullest), 0));
+  } else {
+    last = s_last;
+  }
+  if (fullest > static_cast<uint32_t>(kMaxPerBucket)) {
+    radix();
     return;
   }
-  const int last = s_last;
 
   // ---- elements of those buckets to their bucket's places (bucket[b] moves from its start to its end) ----
 #pragma unroll 2
-  for (int i4 = tid; i4 < n4; i4 += kThreads) {
+  for (int i4 = beg4 + tid; i4 < end4; i4 += kThreads) {
     const float4 v = get4(i4);
     const float f[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -502,11 +565,20 @@ __global__ void __launch_bounds__(kThreads, (kThreads == 512 && kMaxRounds <= 4)
       if (f[j] == -INFINITY) continue;
       const int b = bucket_of(f[j]);
       if (b <= last)
-        list[atomicAdd(&bucket[b], 1u)] = (static_cast<unsigned long long>(float_to_key(f[j])) << 32) |
-                                          static_cast<unsigned long long>(0xffffffffu - static_cast<uint32_t>(4 * i4 + j));
+      {
+        const unsigned long long e = (static_cast<unsigned long long>(float_to_key(f[j])) << 32) |
+                                     static_cast<unsigned long long>(0xffffffffu - static_cast<uint32_t>(4 * i4 + j));
+        if constexpr (kC > 1) st_cluster_u64(lead_list + atom_add_cluster_u32(lead_bucket + b * 4, 1u) * 8, e);
+        else list[atomicAdd(&bucket[b], 1u)] = e;
+      }
     }
   }
-  __syncthreads();
+  if constexpr (kC > 1) {
+    cluster_sync_all();
+    if (rank != 0) return;
+  } else {
+    __syncthreads();
+  }
 
   // ---- place inside the bucket, output ----
   int32_t* oi = out_idx + static_cast<int64_t>(row) * top_k;
@@ -560,12 +632,41 @@ static int launch_bucket(const float* scores, int64_t rows, int n, int64_t row_s
   const size_t smem = bucket_smem_bytes<kThreads>(cache ? n : 0, kp);
   constexpr int kFew = kThreads == 512 ? 4 : 2, kMany = kThreads == 512 ? 16 : 8;   // rounds of the way out's sort: 2048, 8192 survivors
   const bool small = top_k <= kThreads * kFew;
-  auto kern = cache ? (small ? topk_bucket_kernel<kThreads, true, kFew> : topk_bucket_kernel<kThreads, true, kMany>)
-                    : (small ? topk_bucket_kernel<kThreads, false, kFew> : topk_bucket_kernel<kThreads, false, kMany>);
+  auto kern = cache ? (small ? topk_bucket_kernel<kThreads, true, kFew, 1> : topk_bucket_kernel<kThreads, true, kMany, 1>)
+                    : (small ? topk_bucket_kernel<kThreads, false, kFew, 1> : topk_bucket_kernel<kThreads, false, kMany, 1>);
   cudaError_t e = ensure_dynamic_smem(kern, dev, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
   kern<<<static_cast<unsigned>(rows), kThreads, smem, stream>>>(scores, row_stride, n, limits, top_k, kp, out_idx, out_val);
   return static_cast<int>(cudaGetLastError());
+}
+
+// A cluster of kC CTAs of 512 threads per row.
+template <int kC>
+static int launch_bucket_cluster(const float* scores, int64_t rows, int n, int64_t row_stride, const int32_t* limits, int top_k, int kp,
+                                 int32_t* out_idx, float* out_val, int dev, cudaStream_t stream) {
+  const int slice = ((n + 3) / 4 + kC - 1) / kC * 4;
+  // (the way out streams its row: it needs no room for it)
+  auto bytes = [&](int kept) {
+    const size_t own = bucket_smem_bytes<512>(kept, kp), radix = radix_smem_bytes<512>(0, kp);
+    return own > radix ? own : radix;
+  };
+  const bool cache = bytes(slice) <= topk::kMaxSmemBytes / 2;   // two CTAs per SM
+  const size_t smem = bytes(cache ? slice : 0);
+  auto kern = top_k <= 2048 ? (cache ? topk_bucket_kernel<512, true, 4, kC> : topk_bucket_kernel<512, false, 4, kC>)
+                            : (cache ? topk_bucket_kernel<512, true, 16, kC> : topk_bucket_kernel<512, false, 16, kC>);
+  cudaError_t e = ensure_dynamic_smem(kern, dev, static_cast<int>(smem));
+  if (e != cudaSuccess) return static_cast<int>(e);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(rows * kC));
+  cfg.blockDim = dim3(512);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = kC; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, scores, row_stride, n, limits, top_k, kp, out_idx, out_val));
 }
 
 int launch_topk_select(const float* scores, int64_t rows, int n, int64_t row_stride, const int32_t* limits, int top_k,
@@ -581,7 +682,15 @@ int launch_topk_select(const float* scores, int64_t rows, int n, int64_t row_str
   cudaError_t e = current_device_sms(&dev, &sms);
   if (e != cudaSuccess) return static_cast<int>(e);
   if (ordered) {
-    // rows that leave SMs idle anyway get twice the threads
+    // Few rows that one CTA cannot keep in shared memory (more than about 47 k): a cluster per row, as long as the clusters are
+    // resident at once.  49152 -> 2048: 1 row 20.8 -> 12.3 us, 32 rows 21.5 -> 16.3, 60 rows 21.6 -> 18.4; 4 rows of 131072 45.4 ->
+    // 16.5.  Shorter rows do not repay the cluster's barriers and remote atomics (32 rows of 16384: 9.4 -> 17.2).
+    const bool kept = bucket_smem_bytes<1024>(n, kp) <= topk::kMaxSmemBytes;
+    if (!kept && rows * 8 <= 2 * sms)
+      return launch_bucket_cluster<8>(scores, rows, n, row_stride, limits, top_k, kp, out_idx, out_val, dev, stream);
+    if (!kept && rows * 4 <= 2 * sms)
+      return launch_bucket_cluster<4>(scores, rows, n, row_stride, limits, top_k, kp, out_idx, out_val, dev, stream);
+    // other rows that leave SMs idle get twice the threads
     return rows <= sms ? launch_bucket<1024>(scores, rows, n, row_stride, limits, top_k, kp, out_idx, out_val, dev, stream)
                        : launch_bucket<512>(scores, rows, n, row_stride, limits, top_k, kp, out_idx, out_val, dev, stream);
   }
