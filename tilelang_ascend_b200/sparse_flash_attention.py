@@ -56,7 +56,7 @@ def sparse_mla_fwd_raw(q, kv, indices, *, sm_scale: float, q_start: int, causal:
     indices [B,S,1,topk] int32.  Returns (out, lse-or-None).
 
     nsplit: None = let the library decide whether the keys of every query are split over several work units (it does for
-    D=576 / dv=512 calls with fewer queries than SM pairs, e.g. decode of a few sequences); 1 = never; n > 1 = n shares.
+    D=576 / dv=512 calls with fewer queries than SM pairs -- than SMs for at most 64 heads --, e.g. decode of a few sequences); 1 = never; n > 1 = n shares.
     The fp32 workspace of a split call is owned here (one per device and stream, reused between calls), as the reference's
     adapter owns its kernels' workspaces (tilelang/jit/adapter/cython/cython_wrapper.pyx:98-137).
 
