@@ -361,3 +361,40 @@ def test_lengths_known_to_the_device_or_the_host(where, monkeypatch):
     with pytest.raises(ValueError):
         call((77, nb * bs + 1, 3))
     check_status()
+
+
+@pytest.mark.parametrize("N1", [24, 32, 48])
+@pytest.mark.parametrize("paged", [True, False])
+def test_lengths_beyond_the_row_write_nothing_behind_it(N1, paged):
+    """Lengths that the host has not checked (they live on the device) and that exceed the table or the key tensor: the rows end at
+    their width -- same answer as with the lengths clipped, on both kernels (24 and 48 heads: CUDA cores) -- and what lies behind the
+    workspace stays as it was."""
+    import tilelang_ascend_b200 as dsa
+    B, S1, bs, nb, K = 3, 2, 16, 9, 32
+    n = bs * nb
+    q, k, w = orc.make_indexer_inputs(B, S1, n, N1, 128, seed=N1)
+    q, w = q.cuda(), w.cuda()
+    table = None
+    if paged:
+        table = torch.randperm(B * nb, generator=torch.Generator().manual_seed(3)).to(torch.int32).view(B, nb)
+        pool = torch.empty((B * nb, bs, 1, 128), dtype=k.dtype)
+        pool[table.long().view(-1)] = k.view(B * nb, bs, 1, 128)
+        k, table = pool, table.cuda()
+    k = k.cuda()
+    need = int(dsa._lib.load().dsa_lightning_indexer_workspace_bytes(B, S1, n))
+    ql = torch.full((B,), S1, dtype=torch.int32, device="cuda")
+
+    def call(lengths):
+        guarded = torch.full((need + 4096,), 0x5a, dtype=torch.uint8, device="cuda")
+        idx, _ = dsa.lightning_indexer_raw(q, k, w, sparse_count=K, sparse_mode=0, q_len_b=ql, block_table=table, workspace=guarded[:need],
+                                           k_len_b=torch.tensor(lengths, dtype=torch.int32, device="cuda"))
+        check_status()
+        assert bool((guarded[need:] == 0x5a).all())
+        return idx
+
+    assert torch.equal(call((n + 1, n - 5, n + 37)), call((n, n - 5, n)))
+    if paged:
+        with pytest.raises(ValueError, match="covers"):
+            dsa.lightning_indexer(q, k, w, actual_seq_lengths_key=torch.tensor((7, 9, n + 3), dtype=torch.int32, device="cuda"), block_table=table,
+                                  layout_key="PA_BSND", sparse_count=K)
+        check_status()

@@ -32,16 +32,19 @@
 
 namespace dsa {
 
+// Keys [0, limit) of row (b, s1) are candidates; *ak_out is the sequence's key count.  Both end at the row's width S2 whatever
+// the lengths say: they come from device memory that the host may not have looked at yet (it checks them after the launch),
+// and every store and key read below is bounded by them.
 __device__ __forceinline__ int indexer_limit(const IndexerParams& p, int b, int s1, int* ak_out) {
   const int aq = p.q_len_b ? p.q_len_b[b] : p.S1;
   const int ak = p.k_len_b ? p.k_len_b[b] : p.S2;
-  *ak_out = ak;
+  *ak_out = min(ak, p.S2);
   if (s1 >= aq || ak <= 0) return 0;
   if (p.sparse_mode == 3) {
-    const int cl = ak - aq + s1 + 1;
-    return cl > 0 ? (cl < ak ? cl : ak) : ak;
+    const int cl = ak - aq + s1 + 1;   // (from the lengths as given: the causal rule counts from their ends)
+    return min(cl > 0 ? (cl < ak ? cl : ak) : ak, p.S2);
   }
-  return ak;
+  return min(ak, p.S2);
 }
 
 namespace itc {
