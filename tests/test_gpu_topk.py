@@ -167,3 +167,49 @@ def test_bucket_select_is_exact(rows, n, top_k):
         got = dsa.topk_select_raw(wide[:, :n], top_k).cpu().numpy()
         assert np.array_equal(got, orc.topk_select(x, top_k))
     check_status()
+
+
+def _crowded(kind: str, rows: int, n: int, rng) -> np.ndarray:
+    x = rng.standard_normal((rows, n)).astype(np.float32)
+    if kind == "masked":                    # a finite mask value; in the last row most entries, so that masked ones are selected
+        x[rng.random((rows, n)) < 0.3] = np.float32(-1e9)
+        x[-1, rng.random(n) < 0.9] = np.float32(-1e4)
+    elif kind == "outlier":
+        x[:, n // 3] = np.float32(3e4)
+        x[0, n // 2] = np.inf
+    elif kind == "exp":
+        x = np.exp(5 * x).astype(np.float32)
+    elif kind == "quantised":               # a few values, many ties each; zeros of both signs
+        x = (np.round(x * 4) / 4).astype(np.float32)
+    elif kind == "equal":
+        x[:] = np.float32(1.5)
+    elif kind == "clamped":                 # half of the row at its largest value, a few just below it: one crowded fine bucket
+        x = np.minimum(x, np.float32(0.1)).astype(np.float32)
+        x[:, ::n // 7] = np.float32(0.0999)
+    elif kind == "narrow":                  # a few ulps around 1000 beside a far value
+        x = (np.float32(1000.0) + np.float32(1e-4) * x).astype(np.float32)
+        x[:, 5] = np.float32(-1e6)
+    return x
+
+
+@pytest.mark.parametrize("kind", ["masked", "outlier", "exp", "quantised", "equal", "clamped", "narrow"])
+@pytest.mark.parametrize("rows,n,top_k", [(3, 300, 200), (5, 4096, 2048), (200, 4099, 2048), (2, 20000, 8192), (160, 9000, 4096), (2, 49152, 2048),
+                                          (40, 50001, 700), (1, 131072, 2048), (2, 70003, 8192), (301, 2048, 65), (38, 49152, 4096)])
+def test_crowded_rows_are_exact(kind, rows, n, top_k):
+    """Rows whose values crowd into few buckets, over both thread counts, clusters of 8 and 4 CTAs (which then share the radix select), kept
+    and streamed rows: the survivors' order comes from the second level of buckets or from the radix sort; index arrays and values
+    equal the oracle's exactly, the unordered form selects the same sets."""
+    import tilelang_ascend_b200 as dsa
+    rng = np.random.default_rng(n + top_k + len(kind))
+    x = _crowded(kind, rows, n, rng)
+    lim = rng.integers(0, n + 1, size=rows).astype(np.int32)
+    lim[0] = n
+    for limits in (None, lim):
+        got, val = _run(x, top_k, limits, values=True)
+        ref, ref_val = orc.topk_select(x, top_k, limits, return_values=True)
+        assert np.array_equal(got, ref)
+        assert np.array_equal(val, ref_val)
+    sets = dsa.topk_select_raw(torch.from_numpy(x).cuda(), top_k, ordered=False).cpu().numpy()
+    ref = orc.topk_select(x, top_k)
+    assert np.array_equal(np.sort(sets, axis=1), np.sort(ref, axis=1))
+    check_status()
