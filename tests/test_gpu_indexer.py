@@ -398,3 +398,27 @@ def test_lengths_beyond_the_row_write_nothing_behind_it(N1, paged):
             dsa.lightning_indexer(q, k, w, actual_seq_lengths_key=torch.tensor((7, 9, n + 3), dtype=torch.int32, device="cuda"), block_table=table,
                                   layout_key="PA_BSND", sparse_count=K)
         check_status()
+
+
+@pytest.mark.parametrize("N1", [8, 64])
+def test_block_table_much_wider_than_the_sequences(N1):
+    """Score rows as wide as the table: chunks share the tiles that a sequence has (none, less than one, a few chunks', most of the
+    row's), and give the indices of a launch at the longest length."""
+    import tilelang_ascend_b200 as dsa
+    bs, width, K = 128, 70016, 300
+    lens = (0, 1, 129, 1024, 1025, 9000, 65000)
+    B, nb = len(lens), width // bs
+    g = torch.Generator(device="cuda").manual_seed(N1)
+    table = (torch.randperm(B * nb, generator=g, device="cuda") % 600).to(torch.int32).view(B, nb).contiguous()
+    pool = torch.randn((600, bs, 1, 128), generator=g, device="cuda").to(torch.bfloat16)
+    q = torch.randn((B, 1, N1, 128), generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.rand((B, 1, N1), generator=g, device="cuda") / N1
+    aq = torch.ones((B,), dtype=torch.int32, device="cuda")
+    for n in (B, B - 1):   # with and without the long sequence
+        ak = torch.tensor(lens[:n], dtype=torch.int32, device="cuda")
+        kw = dict(sparse_count=K, sparse_mode=3, q_len_b=aq[:n], k_len_b=ak, block_table=table[:n])
+        wide = dsa.lightning_indexer_raw(q[:n], pool, w[:n], **kw)[0]
+        exact = dsa.lightning_indexer_raw(q[:n], pool, w[:n], max_keys=max(lens[:n]), **kw)[0]
+        check_status()
+        assert torch.equal(wide, exact)
+        assert [int((wide[b] >= 0).sum()) for b in range(n)] == [min(x, K) for x in lens[:n]]

@@ -54,6 +54,7 @@ constexpr uint32_t kKStageBytes = 2 * kKeys * 128; // 32768
 constexpr int kEpilogueWarps = 8;                  // warp w: keys 32 (w & 3) .. +31 of a tile
 constexpr int kMmaWarp = 8;
 constexpr int kThreads = 416;                      // 8 reduce warps, the MMA warp, 4 producer warps
+constexpr int kMinTiles = 8;                       // key tiles that are worth a CTA (its start-up costs about two tiles' time)
 // kN = (queries x heads) per CTA = UMMA N.  256 is the prefill shape: one CTA per SM, the two groups of four reduce warps
 // take half of the queries of every tile each.  With few queries (decode) the columns of queries that do not exist would
 // cost as much as real ones, so the smallest of 64, 128 and 256 that holds all S1 x N1 rows is taken; the narrow shapes
@@ -98,10 +99,10 @@ __global__ void __launch_bounds__(itc::kThreads, itc::Cfg<kN>::kCtas)
   int* start_status = reinterpret_cast<int*>(bars + 11);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // Work unit = (chunk of tiles_per_cta key tiles, batch entry, block of queries).  First chunks come first: the last ones
-  // are empty for the shorter sequences of a ragged batch.
+  // Work unit = (chunk of key tiles, batch entry, block of queries).  First chunks come first: the last ones are empty for
+  // sequences of few tiles.
   const int nqb = (p.S1 + QB - 1) / QB;
-  const int chunk = blockIdx.x / (p.B * nqb), unit = blockIdx.x - chunk * (p.B * nqb);
+  const int chunk = blockIdx.x / (p.B * nqb), unit = blockIdx.x - chunk * (p.B * nqb), chunks = gridDim.x / (p.B * nqb);
   const int b = unit / nqb;
   const int qb = nqb - 1 - (unit - b * nqb);  // late (long) query blocks first
   const int q0 = qb * QB;
@@ -116,11 +117,15 @@ __global__ void __launch_bounds__(itc::kThreads, itc::Cfg<kN>::kCtas)
     const int s1 = q0 + i;
     if (s1 < p.S1) { const int l = indexer_limit(p, b, s1, &ak); max_lim = l > max_lim ? l : max_lim; }
   }
-  // this CTA's key tiles: [tile0, tile0 + ntiles_mma) are scored, those up to tile0 + ntiles_all only filled with -inf
-  const int tile0 = chunk * p.tiles_per_cta;
+  // This CTA's key tiles: [tile0, tile0 + ntiles_mma) are scored, those up to tile0 + ntiles_all only filled with -inf.  The chunks
+  // share the tiles that THIS sequence has, not those of the row's width: a block table is usually wider than its sequences,
+  // and the host does not know them (32 sequences of up to 4096 keys in a table for 131072, scores + selector: 41 us with chunks
+  // of the table's width, 35 with these; 32 under a table for 4096).
   const int tiles_scored = (max_lim + kKeys - 1) / kKeys, tiles_total = p.fill_masked ? (p.S2 + kKeys - 1) / kKeys : tiles_scored;
-  const int ntiles_mma = max(0, min(tiles_scored - tile0, p.tiles_per_cta));
-  const int ntiles_all = max(0, min(tiles_total - tile0, p.tiles_per_cta));
+  const int tiles_per_cta = max(kMinTiles, (tiles_total + chunks - 1) / chunks);
+  const int tile0 = chunk * tiles_per_cta;
+  const int ntiles_mma = max(0, min(tiles_scored - tile0, tiles_per_cta));
+  const int ntiles_all = max(0, min(tiles_total - tile0, tiles_per_cta));
   if (p.limits && chunk == 0 && tid < QB && q0 + tid < p.S1) {
     int dummy;
     p.limits[static_cast<int64_t>(b) * p.S1 + q0 + tid] = indexer_limit(p, b, q0 + tid, &dummy);
@@ -392,14 +397,14 @@ static int launch_indexer_tc_shape(const IndexerParams& p_in, cudaStream_t strea
   constexpr int QB = kN / N1;
   const long long units = static_cast<long long>(p.B) * ((p.S1 + QB - 1) / QB);
   // Keys are split into chunks, one CTA each, while the CTAs are fewer than kRounds rounds of the chip (ragged lengths even
-  // out over several rounds), but a chunk keeps at least kMinTiles tiles (a CTA's start-up costs about two tiles' time).
-  constexpr int kRounds = kN == 256 ? 2 : 4, kMinTiles = 8;
+  // out over several rounds), but a chunk keeps at least kMinTiles tiles.
+  constexpr int kRounds = kN == 256 ? 2 : 4;
   const int tiles = (p.S2 + itc::kKeys - 1) / itc::kKeys;
   long long chunks = (static_cast<long long>(kRounds) * sms * itc::Cfg<kN>::kCtas + units - 1) / units;
-  if (chunks > tiles / kMinTiles) chunks = tiles / kMinTiles;
+  if (chunks > tiles / itc::kMinTiles) chunks = tiles / itc::kMinTiles;
   if (chunks < 1) chunks = 1;
-  p.tiles_per_cta = static_cast<int>((tiles + chunks - 1) / chunks);
-  chunks = (tiles + p.tiles_per_cta - 1) / p.tiles_per_cta;
+  const long long per_chunk = (tiles + chunks - 1) / chunks;
+  chunks = (tiles + per_chunk - 1) / per_chunk;   // (no empty ones for a sequence of the row's width)
   alignas(64) CUtensorMap kmap;
   memset(&kmap, 0, sizeof(kmap));
   // DSA_INDEXER_NO_TMA=1 in the environment forces the cp.async producers (used by the tests to cover that path)

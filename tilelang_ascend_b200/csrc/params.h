@@ -86,7 +86,6 @@ struct IndexerParams {
   const int32_t* block_table;
   int block_size, max_blocks, num_blocks;
   int box_rows;               // set by the launcher: rows per TMA box of a paged cache
-  int tiles_per_cta;          // set by the launcher: key tiles per CTA of the tensor-core kernel
 };
 
 // Block-sparse indexer logits (HISA).
