@@ -213,3 +213,17 @@ def test_crowded_rows_are_exact(kind, rows, n, top_k):
     ref = orc.topk_select(x, top_k)
     assert np.array_equal(np.sort(sets, axis=1), np.sort(ref, axis=1))
     check_status()
+
+
+@pytest.mark.parametrize("rows,n,top_k", [(8, 131072, 2048), (50, 60001, 700), (8, 200003, 8192)])
+def test_short_rows_of_a_cluster_launch(rows, n, top_k):
+    """Rows as wide as a block table whose candidates fit one CTA of the row's cluster are that CTA's alone: limits on both sides of a
+    slice, crowded rows among them."""
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((rows, n)).astype(np.float32)
+    x[::3] = np.round(x[::3] * 4) / 4
+    c = 8 if rows * 8 <= 296 else 4
+    piece = (-(-n // 4) + c - 1) // c * 4
+    lim = rng.integers(0, n, size=rows).astype(np.int32)
+    lim[:8] = (-1, 0, 1, piece - 1, piece, piece + 1, piece // 2, n)
+    assert np.array_equal(_run(x, top_k, lim), orc.topk_select(x, top_k, lim))

@@ -28,6 +28,9 @@ constexpr int kSelectThreads = 512;               // 4 rows (CTAs) per SM hide e
 constexpr int kBuckets = 4096;
 constexpr int kMaxPerBucket = 96;                 // fuller buckets: radix select instead (bucket_sort: a second level of buckets)
 constexpr size_t kMaxSmemBytes = 220 * 1024;       // rows whose keys do not fit are streamed from global memory
+constexpr size_t kMaxClusterSmemBytes = 105 * 1024;   // dynamic, of a CTA of a cluster: two of them per SM, with 8 KB static each
+// candidates of a row of n that each of c CTAs takes at most: whole groups of four
+__host__ __device__ constexpr int cluster_slice(int n, int c) { return ((n + 3) / 4 + c - 1) / c * 4; }
 }  // namespace topk
 
 __device__ __forceinline__ uint32_t float_to_key(float f) {
@@ -624,12 +627,11 @@ __global__ void __launch_bounds__(topk::kSelectThreads, 4)
 // range into the first CTA's, and put the elements into its list; the rest is the first CTA's work.
 // kCache: the row (slice) stays in shared memory after the first pass; longer rows are read three times (from L2).
 template <int kThreads, bool kCache, int kMaxRounds, int kC>
-__global__ void __launch_bounds__(kThreads, (kThreads == 512 && kMaxRounds <= 4) ? 3 : 1)
-    topk_bucket_kernel(const float* __restrict__ scores, int64_t row_stride, int n_all, const int32_t* __restrict__ limits, int top_k, int kp,
-                       int32_t* __restrict__ out_idx, float* __restrict__ out_val) {
+__device__ __forceinline__ void bucket_select_row(uint8_t* smem_raw, const int row, const float* __restrict__ scores, int64_t row_stride, int n_all,
+                                                  const int32_t* __restrict__ limits, int top_k, int kp, int32_t* __restrict__ out_idx,
+                                                  float* __restrict__ out_val) {
   using namespace topk;
   constexpr int kWarps = kThreads / 32, kPer = kBuckets / kThreads;
-  extern __shared__ __align__(16) uint8_t smem_raw[];
   uint32_t* bucket = reinterpret_cast<uint32_t*>(smem_raw);                                    // [kBuckets] counts, then ends
   unsigned long long* list = reinterpret_cast<unsigned long long*>(smem_raw + kBuckets * 4);   // [kp + kMaxPerBucket]
   float* cache = reinterpret_cast<float*>(list + kp + kMaxPerBucket);                          // [n rounded up to 4]
@@ -639,7 +641,6 @@ __global__ void __launch_bounds__(kThreads, (kThreads == 512 && kMaxRounds <= 4)
   __shared__ uint32_t s_fullest;
   __shared__ float s_range[2];   // this CTA's minimum and maximum (kC > 1)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int row = blockIdx.x / kC;
   const uint32_t rank = kC > 1 ? cluster_ctarank() : 0u;
   const float* x = scores + static_cast<int64_t>(row) * row_stride;
   int n = limits ? limits[row] : n_all;
@@ -847,6 +848,25 @@ __global__ void __launch_bounds__(kThreads, (kThreads == 512 && kMaxRounds <= 4)
   }
 }
 
+// A cluster's row whose candidates fit the first CTA's slice is that CTA's alone, the others leave: score rows are as wide as the
+// caller's block table, the sequence may be short (64 sequences of up to 3000 keys in a table for 131072, scores + selector:
+// 36 -> 29 us; 26 under a table for 3000).
+template <int kThreads, bool kCache, int kMaxRounds, int kC>
+__global__ void __launch_bounds__(kThreads, (kThreads == 512 && kMaxRounds <= 4) ? 3 : 1)
+    topk_bucket_kernel(const float* __restrict__ scores, int64_t row_stride, int n, const int32_t* __restrict__ limits, int top_k, int kp,
+                       int32_t* __restrict__ out_idx, float* __restrict__ out_val) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  const int row = blockIdx.x / kC;
+  if constexpr (kC > 1) {
+    if (limits && limits[row] <= topk::cluster_slice(n, kC)) {
+      if (cluster_ctarank() == 0)
+        bucket_select_row<kThreads, kCache, kMaxRounds, 1>(smem_raw, row, scores, row_stride, n, limits, top_k, kp, out_idx, out_val);
+      return;
+    }
+  }
+  bucket_select_row<kThreads, kCache, kMaxRounds, kC>(smem_raw, row, scores, row_stride, n, limits, top_k, kp, out_idx, out_val);
+}
+
 // Shared memory of the kernel that keeps a row's keys (n > 0) or of the streaming kernel (n = 0).
 template <int kThreads>
 static size_t radix_smem_bytes(int n, int kp) {
@@ -889,15 +909,11 @@ static int launch_bucket(const float* scores, int64_t rows, int n, int64_t row_s
 // A cluster of kC CTAs of 512 threads per row.
 template <int kC>
 static int launch_bucket_cluster(const float* scores, int64_t rows, int n, int64_t row_stride, const int32_t* limits, int top_k, int kp,
-                                 int32_t* out_idx, float* out_val, int dev, cudaStream_t stream) {
-  const int slice = ((n + 3) / 4 + kC - 1) / kC * 4;
-  // (the way out streams its row: it needs no room for it)
-  auto bytes = [&](int kept) {
-    const size_t own = bucket_smem_bytes<512>(kept, kp), radix = radix_smem_bytes<512>(0, kp);
-    return own > radix ? own : radix;
-  };
-  const bool cache = bytes(slice) <= topk::kMaxSmemBytes / 2;   // two CTAs per SM
-  const size_t smem = bytes(cache ? slice : 0);
+                                 int32_t* out_idx, float* out_val, int dev, int sms, cudaStream_t stream) {
+  const int slice = topk::cluster_slice(n, kC);
+  const size_t most = rows * kC <= sms ? topk::kMaxSmemBytes : topk::kMaxClusterSmemBytes;   // one or two CTAs per SM
+  const bool cache = bucket_smem_bytes<512>(slice, kp) <= most;
+  const size_t smem = bucket_smem_bytes<512>(cache ? slice : 0, kp);   // (a row that one CTA takes alone fits a slice)
   auto kern = top_k <= 2048 ? (cache ? topk_bucket_kernel<512, true, 4, kC> : topk_bucket_kernel<512, false, 4, kC>)
                             : (cache ? topk_bucket_kernel<512, true, 16, kC> : topk_bucket_kernel<512, false, 16, kC>);
   cudaError_t e = ensure_dynamic_smem(kern, dev, static_cast<int>(smem));
@@ -929,9 +945,9 @@ int launch_topk_select(const float* scores, int64_t rows, int n, int64_t row_str
     // 16.5.  Shorter rows do not repay the cluster's barriers and remote atomics (32 rows of 16384: 9.4 -> 17.2).
     const bool kept = bucket_smem_bytes<1024>(n, kp) <= topk::kMaxSmemBytes;
     if (!kept && rows * 8 <= 2 * sms)
-      return launch_bucket_cluster<8>(scores, rows, n, row_stride, limits, top_k, kp, out_idx, out_val, dev, stream);
+      return launch_bucket_cluster<8>(scores, rows, n, row_stride, limits, top_k, kp, out_idx, out_val, dev, sms, stream);
     if (!kept && rows * 4 <= 2 * sms)
-      return launch_bucket_cluster<4>(scores, rows, n, row_stride, limits, top_k, kp, out_idx, out_val, dev, stream);
+      return launch_bucket_cluster<4>(scores, rows, n, row_stride, limits, top_k, kp, out_idx, out_val, dev, sms, stream);
     // other rows that leave SMs idle get twice the threads
     return rows <= sms ? launch_bucket<1024>(scores, rows, n, row_stride, limits, top_k, kp, out_idx, out_val, dev, stream)
                        : launch_bucket<512>(scores, rows, n, row_stride, limits, top_k, kp, out_idx, out_val, dev, stream);
