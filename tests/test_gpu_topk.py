@@ -215,10 +215,10 @@ def test_crowded_rows_are_exact(kind, rows, n, top_k):
     check_status()
 
 
-@pytest.mark.parametrize("rows,n,top_k", [(8, 131072, 2048), (50, 60001, 700), (8, 200003, 8192)])
+@pytest.mark.parametrize("rows,n,top_k", [(8, 131072, 2048), (50, 60001, 700), (8, 200003, 8192), (9, 382400, 2048)])
 def test_short_rows_of_a_cluster_launch(rows, n, top_k):
     """Rows as wide as a block table whose candidates fit one CTA of the row's cluster are that CTA's alone: limits on both sides of a
-    slice, crowded rows among them."""
+    slice, crowded rows among them.  (382400: a slice that just fits the shared memory of a CTA which has its SM alone.)"""
     rng = np.random.default_rng(n)
     x = rng.standard_normal((rows, n)).astype(np.float32)
     x[::3] = np.round(x[::3] * 4) / 4

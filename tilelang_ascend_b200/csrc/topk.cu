@@ -28,7 +28,8 @@ constexpr int kSelectThreads = 512;               // 4 rows (CTAs) per SM hide e
 constexpr int kBuckets = 4096;
 constexpr int kMaxPerBucket = 96;                 // fuller buckets: radix select instead (bucket_sort: a second level of buckets)
 constexpr size_t kMaxSmemBytes = 220 * 1024;       // rows whose keys do not fit are streamed from global memory
-constexpr size_t kMaxClusterSmemBytes = 105 * 1024;   // dynamic, of a CTA of a cluster: two of them per SM, with 8 KB static each
+// dynamic, of a CTA of a cluster, beside 8 KB static: two of them per SM (228 KB), or one that has the SM alone (227 KB)
+constexpr size_t kMaxClusterSmemBytes = 105 * 1024, kMaxLoneClusterSmemBytes = 219 * 1024;
 // candidates of a row of n that each of c CTAs takes at most: whole groups of four
 __host__ __device__ constexpr int cluster_slice(int n, int c) { return ((n + 3) / 4 + c - 1) / c * 4; }
 }  // namespace topk
@@ -617,8 +618,8 @@ __global__ void __launch_bounds__(topk::kSelectThreads, 4)
 // places, and an element's final place is its bucket's start plus the number of elements of the same bucket in front of it
 // (larger key, or equal key and lower index): a handful of comparisons, no sort, no search inside the threshold's bucket.
 // Rows whose values crowd (more than kMaxPerBucket in a bucket that is needed, a range that is zero or not finite) take the
-// radix select; by then they have cost a range pass and a histogram, so that what follows must be faster than the radix select
-// and four-pass sort alone (start below).  Whole calls, us, radix alone -> here: 4096 rows of 8192 -> 2048 with a finite mask 375 -> 268, with an
+// radix select; by then they have cost a range pass and a histogram, which its sort by buckets has to win back against the
+// radix select with a four-pass sort alone.  Whole calls, us, that one -> here: 4096 rows of 8192 -> 2048 with a finite mask 375 -> 268, with an
 // outlier 375 -> 289, exp(3 x) 377 -> 274, rounded to quarters 299 -> 305 (the worst kind: mostly ties, 0.96 to 1.0 of radix
 // alone over the sizes tried); 32 rows of 49152 with a finite mask 63 -> 42, 300 rows 190 -> 174.  Rows that do not crowd: 4096
 // rows of up to 8192 -> 2048: 380 -> 112 us; 64 rows of 4096 -> 2048, whole call: 22.5 -> 15.0 us.
@@ -911,7 +912,7 @@ template <int kC>
 static int launch_bucket_cluster(const float* scores, int64_t rows, int n, int64_t row_stride, const int32_t* limits, int top_k, int kp,
                                  int32_t* out_idx, float* out_val, int dev, int sms, cudaStream_t stream) {
   const int slice = topk::cluster_slice(n, kC);
-  const size_t most = rows * kC <= sms ? topk::kMaxSmemBytes : topk::kMaxClusterSmemBytes;   // one or two CTAs per SM
+  const size_t most = rows * kC <= sms ? topk::kMaxLoneClusterSmemBytes : topk::kMaxClusterSmemBytes;
   const bool cache = bucket_smem_bytes<512>(slice, kp) <= most;
   const size_t smem = bucket_smem_bytes<512>(cache ? slice : 0, kp);   // (a row that one CTA takes alone fits a slice)
   auto kern = top_k <= 2048 ? (cache ? topk_bucket_kernel<512, true, 4, kC> : topk_bucket_kernel<512, false, 4, kC>)
