@@ -578,10 +578,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pr::kThreads, 1) spa
         }
         qslots += 2;
       }
-      // Lane l looks up key 8 pw + (l & 7) of this CTA's 32 keys of a tile.  The look-up is a chain of two loads that may each
-      // miss every cache (index list, block table): the index is loaded two tiles ahead and the row number formed one tile
-      // ahead, so that neither latency sits in the per-tile period of these warps (paged decode of 64 sequences, whole call:
-      // 78.5 -> 69.8 us; prefill, whose lists come from L2, unchanged).
+      // Lane l looks up key 8 pw + (l & 7) of this CTA's 32 keys of a tile.  The index is loaded one tile ahead, so that its
+      // latency (a miss of every cache in decode) does not sit in the per-tile period of these warps; the row number, which a
+      // block table gives from a cached line, is formed in its own tile.  Paged decode of 64 sequences, whole call: no look-ahead
+      // 72.1 us, this 61.6, row numbers one tile and indices two tiles ahead 61.6 -- but that form's extra state slows the
+      // prefill (4096 queries, 128 heads, full clock): 1.669, 1.668 and 1.681 ms.
       auto load_idx = [&](int it) {
         const int slot = it < nvt ? tile_list[qp * kMaxTiles + it] * kBK + static_cast<int>(rank) * kKeys + pw * 8 + (lane & 7) : p.topk;
         return slot < p.topk ? __ldg(ctx.idx_row + slot) : -1;
@@ -596,13 +597,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pr::kThreads, 1) spa
         return static_cast<int>(kv_row(p, ctx.b, idx));
       };
       int idx_next = load_idx(0);
-      int row_next = row_of(idx_next);
-      idx_next = load_idx(1);
       for (int it = 0; it < nvt; ++it, ++g) {
         const int s = (g + qslots) % kStages;
-        const int my_row = row_next;
-        row_next = row_of(idx_next);
-        idx_next = load_idx(it + 2);
+        const int my_row = row_of(idx_next);
+        idx_next = load_idx(it + 1);
         if (g + qslots >= kStages && ok) ok = mbar_wait<true>(bar(kBarKvEmpty + s), (((g + qslots) / kStages) + 1) & 1, p.status);
         if (!ok) continue;
         const uint32_t stage = sBase + s * kStageBytes;
