@@ -67,9 +67,9 @@ int dsa_topk_select(const float* scores, int64_t rows, int64_t n, int64_t row_st
                     int32_t top_k, int32_t* out_idx, float* out_val, void* stream);
 
 /* dsa_topk_select without the final sort: the same SET of top_k indices per row (the same lowest-index tie rule at the
- * threshold), written in ASCENDING INDEX order instead of descending score order.  For consumers that only need the set --
- * the sparse attention that follows the indexer -- at about half the selector's time.  No reference counterpart (the reference
- * selector always sorts). */
+ * threshold), written in ASCENDING INDEX order instead of descending score order, the order in which the row gather of the
+ * sparse attention that follows is most local.  Not faster than dsa_topk_select, whose value buckets need no sort.  No
+ * reference counterpart (the reference selector always sorts). */
 int dsa_topk_select_unordered(const float* scores, int64_t rows, int64_t n, int64_t row_stride, const int32_t* limits,
                               int32_t top_k, int32_t* out_idx, float* out_val, void* stream);
 
@@ -158,17 +158,17 @@ int dsa_sparse_mla_fwd(const void* q, const void* kv, const int32_t* indices, vo
                        int32_t max_blocks, int32_t impl, void* stream);
 
 /* The same forward with the keys of every query split over `nsplit` work units (tensor-core kernel only: D = 576,
- * DV = 512): for calls with fewer (query, block of 128 heads) items than SM pairs -- decode with a handful of
- * sequences per GPU -- where one unit per query would leave most of the GPU idle.  Each unit writes a normalised
- * partial output and its log-sum-exp into `workspace` (fp32, size from dsa_sparse_mla_fwd_splitkv_workspace_bytes,
+ * DV = 512): for calls with fewer (query, block of 128 heads) items than SM pairs (at most 64 heads and 2048 keys: fewer
+ * queries than SMs) -- decode with a handful of sequences per GPU -- where one unit per query would leave most of the GPU
+ * idle.  Each unit writes a normalised partial output and its log-sum-exp into `workspace` (fp32, size from dsa_sparse_mla_fwd_splitkv_workspace_bytes,
  * 16-byte aligned, owned by the caller); a second kernel on the same stream combines them into out / lse.
  * nsplit = 1 is dsa_sparse_mla_fwd with impl = DSA_IMPL_TENSOR_CORE; dsa_sparse_mla_fwd_splitkv_nsplit suggests a
  * value for the current device (1 = do not split).  Queries that do not exist (q_len_b) get out = 0, lse = -inf.
  * Replaces the same reference kernels as dsa_sparse_mla_fwd (their decode shape:
  * bench_sfa/sparse_flash_attn_pa_no_cv_pipeline.py:384-419, T = 1). */
 /* The forward with only the FIRST split_queries of the B * S queries (memory order) split into nsplit shares each, the
- * others handled whole: for launches whose last round of work units fills the SM pairs only partly (e.g. one GPU's block
- * of a sharded prefill: a persistent kernel reaches the first queries last) -- the split queries' shares then fill that
+ * others handled whole: for launches whose last round of work units fills the SM pairs (at most 64 heads and 2048 keys: the
+ * SMs) only partly (e.g. one GPU's block of a sharded prefill: a persistent kernel reaches the first queries last) -- the split queries' shares then fill that
  * round.  workspace: dsa_sparse_mla_fwd_splitkv_workspace_bytes(1, split_queries, H, DV, nsplit) bytes.  Results of the
  * split queries are combined from fp32 partial results (same tolerance as dsa_sparse_mla_fwd_splitkv, not bit-equal to the
  * unsplit kernel); all other rows are bit-equal to dsa_sparse_mla_fwd. */

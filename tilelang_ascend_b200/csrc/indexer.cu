@@ -16,8 +16,8 @@
 //
 // A batch entry with few queries (decode) takes a narrower B operand, and its keys are split over as many CTAs as fill the
 // chip: one CTA per sequence, 256 columns wide, left 116 of 148 SMs idle and spent three quarters of its reduction on queries
-// that do not exist (32 sequences of up to 49152 paged keys, 64 heads, whole lightning_indexer call with its selector and
-// host reads: 479 -> 214 us; 4096 queries x 8192 keys, whole call: 736 -> 707 us).
+// that do not exist (32 sequences of up to 49152 paged keys, 64 heads, the scores alone: ~390 -> 59 us; 4096 queries x 8192
+// keys, whole call with the selector of that time: 736 -> 707 us).
 //
 // Generic kernel (any D, any N1): CUDA-core fp32.
 #include <cuda.h>

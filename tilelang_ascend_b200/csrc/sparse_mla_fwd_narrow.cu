@@ -30,7 +30,8 @@ namespace nw {
 constexpr int kD = 576, kDV = 512;
 constexpr int kHeads = 64;
 constexpr int kBK = 32;                                // keys per tile
-constexpr int kMaxTiles = 64;                          // topk <= 2048
+// topk <= 2048.  Longer lists keep the pair kernel: not one has been timed here (masks and lists of 8192 keys would fit).
+constexpr int kMaxTiles = 64;
 constexpr int kQTmemChunks = 6;                        // Q dims 0..383 are a tensor-memory operand, the rest stays in shared memory
 constexpr uint32_t kChunk = kBK * 128;                 // 4096: 32 keys x 64 dims, 128-byte swizzle
 constexpr uint32_t kQChunk = kHeads * 128;             // 8192: 64 heads x 64 dims
@@ -396,7 +397,8 @@ __global__ void __launch_bounds__(nw::kThreads, 1) sparse_mla_fwd_narrow_kernel(
       const RowCtx ctx = make_row_ctx(p, bt);
       if (ok) ok = wait_all_idle(kBarInfoFull + qp, (k >> 1) & 1);
       const int nvt = ok ? info[qp] : 0;
-      // lane l looks up key 8 pw + (l & 7); index two tiles ahead, row number one tile ahead (see the pair kernel)
+      // lane l looks up key 8 pw + (l & 7); index two tiles ahead, row number one tile ahead: neither load's latency is in the
+      // warp's per-tile period
       auto load_idx = [&](int it) {
         const int slot = it < nvt ? tile_list[qp * kMaxTiles + it] * kBK + pw * 8 + (lane & 7) : p.topk;
         return slot < p.topk ? __ldg(ctx.idx_row + slot) : -1;

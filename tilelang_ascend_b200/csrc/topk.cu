@@ -620,8 +620,9 @@ __global__ void __launch_bounds__(topk::kSelectThreads, 4)
 // Rows whose values crowd (more than kMaxPerBucket in a bucket that is needed, a range that is zero or not finite) take the
 // radix select; by then they have cost a range pass and a histogram, which its sort by buckets has to win back against the
 // radix select with a four-pass sort alone.  Whole calls, us, that one -> here: 4096 rows of 8192 -> 2048 with a finite mask 375 -> 268, with an
-// outlier 375 -> 289, exp(3 x) 377 -> 274, rounded to quarters 299 -> 305 (the worst kind: mostly ties, 0.96 to 1.0 of radix
-// alone over the sizes tried); 32 rows of 49152 with a finite mask 63 -> 42, 300 rows 190 -> 174.  Rows that do not crowd: 4096
+// outlier 375 -> 289, exp(3 x) 377 -> 274, rounded to quarters 301 -> 308 (the worst kind: few distinct values; 1024 rows of
+// 16384 -> 512: 121 -> 131.  A sample of the row for equal values, looked at before the histogram, makes these two 273 and 110 but
+// rows of distinct values 3 to 7 % slower); 32 rows of 49152 with a finite mask 63 -> 42, 300 rows 190 -> 174.  Rows that do not crowd: 4096
 // rows of up to 8192 -> 2048: 380 -> 112 us; 64 rows of 4096 -> 2048, whole call: 22.5 -> 15.0 us.
 // kC > 1: a cluster of kC CTAs per row, each with a contiguous slice of it (few long rows: one CTA per row leaves most SMs idle
 // and is bound by its own shared-memory atomics).  The CTAs exchange their ranges, sum the histograms bucket range by bucket

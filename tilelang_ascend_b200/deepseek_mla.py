@@ -1,7 +1,7 @@
 """Dense MLA decode behind the reference's three factory signatures
 (examples_experiment/deepseek_mla/): every key of a sequence's latent cache takes part, so each call is the
 sparse forward with the identity index list -- one query token per sequence, non-causal, split over the
-keys when there are fewer sequences than SM pairs.
+keys when there are fewer sequences than SM pairs (at most 64 heads and 2048 keys: than SMs).
 
 * ``mla_decode``            example_mla_decode/example_mla_decode.py:46-92 (dense cache, optional actual length)
 * ``mla_decode_tilelang``   example_mla_decode_paged/example_mla_decode_paged.py:41-131 (paged cache + block table)

@@ -51,8 +51,8 @@ def lightning_indexer_raw(query, key, weights, *, sparse_count: int, sparse_mode
     queries, each with the per-sequence lengths that give its queries the causal limits they have in the whole call
     (dense keys, no caller-owned workspace or lengths, at least as many keys as queries); results are identical.
 
-    ``ordered=False`` leaves the selector's final sort out: the same index SETS, in ascending index order (enough for the
-    sparse attention that consumes them, which does not depend on the order of a query's list).
+    ``ordered=False``: the same index SETS, in ascending index order (the sparse attention that consumes them does not depend
+    on the order of a query's list; this one is the most local for its gather).  The selector is not faster this way.
 
     With ``block_table`` [B, max_blocks] int32, ``key`` is a paged cache [num_blocks, block_size, 1, D] that the kernel
     addresses through the table (no dense copy); ``max_keys`` (default max_blocks * block_size) is the largest logical

@@ -77,8 +77,8 @@ def tail_split_plan(costs, start: int, end: int, units_per_round: int):
 
 def block_time_in_rounds(costs, start: int, end: int, units_per_round: int, tail_split: bool = False) -> int:
     """Time (in the unit of ``costs``) a persistent kernel needs for items [start, end) when it walks them from the last
-    item backwards in rounds of ``units_per_round`` (one item per SM pair and round; every round lasts as long as its most
-    expensive item): the sum over rounds of the largest cost in the round.  ``tail_split``: the last, partly filled round
+    item backwards in rounds of ``units_per_round`` (the items that the GPU works on at once, see :func:`shard_queries`; every
+    round lasts as long as its most expensive item): the sum over rounds of the largest cost in the round.  ``tail_split``: the last, partly filled round
     may be run with its items split into shares (:func:`tail_split_plan`)."""
     import numpy as np
     c = np.asarray(costs)
@@ -141,8 +141,9 @@ def shard_queries(q, indices, rank: int, world: int, s_kv: int, balance: bool = 
     """Query block of this rank for a BSND prefill call: (q_shard, indices_shard, q_start_index_s).
 
     The causal position of local query t is ``q_start_index_s + t`` with ``q_start_index_s = (s_kv - S) + start``.
-    ``balance``: cut by the cost model of :func:`causal_query_costs` instead of by query count; with ``units_per_round``
-    (the GPU's SM pairs: one (query, 128 heads) unit per pair and round) by :func:`shard_ranges_by_rounds`."""
+    ``balance``: cut by the cost model of :func:`causal_query_costs` instead of by query count; with ``units_per_round`` by
+    :func:`shard_ranges_by_rounds`: the queries that the forward works on at once, one per SM for at most 64 heads and lists of
+    at most 2048 keys, one per SM pair otherwise (up to 128 heads)."""
     S = q.shape[1]
     if balance and units_per_round > 0:
         s, e = shard_ranges_by_rounds(causal_query_costs(S, s_kv, indices.shape[-1]), world, units_per_round)[rank]

@@ -16,7 +16,7 @@ def topk_select_raw(scores: torch.Tensor, top_k: int, limits: Optional[torch.Ten
     """scores fp32 [rows, n] (row stride may exceed n) -> int32 [rows, top_k] (+ fp32 values).
 
     Descending score, equal scores by ascending index; -1 / -inf in unused slots.  ``ordered=False``: the same set of
-    indices per row (same tie rule at the threshold) in ascending index order, without the final sort."""
+    indices per row (same tie rule at the threshold) in ascending index order; not the faster form."""
     if scores.dim() != 2 or scores.stride(1) != 1:
         raise ValueError("scores must be 2-dimensional with unit inner stride")
     dev = _check(scores, limits)
